@@ -388,7 +388,6 @@ void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, cha
   j.D = nullptr;
   j.G = nullptr;
   j.Tw = nullptr;
-  j.Dy = nullptr;
   j.On = nullptr;
   j.clip_max = nullptr;
   j.clip = 0;

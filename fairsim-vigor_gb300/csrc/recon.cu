@@ -41,20 +41,20 @@ namespace fsim {
 std::vector<float> fade_vector(int w, int h, int px);
 
 // ---- plan build kernels -------------------------------------------------------------------------
-// conj(OTF(r - k)) mask of one component over its window, quad layout [xl/4][yl][xl%4]:
-// real values for estimated OTFs; complex values (float2) of OTF band `band` for measured
-// ones (OtfProvider.applyOtf(vec, band, kx, ky), S/SimAlgorithm.java:397-403). Table
+// conj(OTF(r - k)) mask of one component over its window, times scale, column by column
+// [xl][yl]: real values for estimated OTFs; complex values (float2) of OTF band `band` for
+// measured ones (OtfProvider.applyOtf(vec, band, kx, ky), S/SimAlgorithm.java:397-403). Table
 // positions in float-float, the reference's double-precision lookup at their boundaries.
 __global__ void k_build_mask(float* __restrict__ mask, int W, int nWin, int Xs, int Ys, double kx, double ky, FShift kf,
-                             const OtfTable* __restrict__ t, int att, int band) {
-  const int xl = blockIdx.x * blockDim.x + threadIdx.x, yl = blockIdx.y;
-  if (xl >= nWin) return;
+                             const OtfTable* __restrict__ t, int att, int band, float scale) {
+  const int yl = blockIdx.x * blockDim.x + threadIdx.x, xl = blockIdx.y;
+  if (yl >= nWin) return;
   int X = (Xs + xl) % W, Y = (Ys + yl) % W;
-  const size_t i = ((size_t)(xl >> 2) * nWin + yl) * 4 + (xl & 3);
+  const size_t i = (size_t)xl * nWin + yl;
   float2 c = make_float2(0.f, 0.f);
   if (!otf_at_fast(*t, band, freq_x(X, W), freq_y(Y, W), kf, kx, ky, att != 0, &c)) c = make_float2(0.f, 0.f);
-  if (t->measured) reinterpret_cast<float2*>(mask)[i] = make_float2(c.x, -c.y);
-  else mask[i] = c.x;
+  if (t->measured) reinterpret_cast<float2*>(mask)[i] = make_float2(scale * c.x, -scale * c.y);
+  else mask[i] = scale * c.x;
 }
 
 // 1/(sum |OTF|^2 + w^2) * apo, quad layout [X/4][Y][X%4], for the columns X < ncols; the
@@ -150,29 +150,23 @@ int Plan::build(cudaStream_t st) {
       win[2 * (a * nC + c)] = xs;
       win[2 * (a * nC + c) + 1] = ys;
     }
-  // The neg component of each pair uses the mirror image of its pos window (columns and
-  // rows), so that pos values can be formed from the neg transforms at (-X, -Y). The pos
-  // window has slack on both sides of the OTF support, so the mirror covers the neg support.
   const int nPair = prm.nr_bands - 1;
-  for (int a = 0; a < nA; a++)
-    for (int b = 1; b <= nPair; b++) {
-      const int cp = 2 * b, cn = 2 * b - 1;
-      win[2 * (a * nC + cn)] = ((W - win[2 * (a * nC + cp)] - nwin + 1) % W + W) % W;
-      win[2 * (a * nC + cn) + 1] = ((W - win[2 * (a * nC + cp) + 1] - nwin + 1) % W + W) % W;
-    }
-  // Nyquist response of each pair's pos component along x and along y:
-  // FFT_N((-1)^n ro[n]) with ro[n] = exp(+2 pi i k (2n+1)/W)/W (k = kx, resp. -ky), i.e.
+  // Response of each pair's neg component to the Nyquist bin, along x over its window's columns
+  // and along y over its rows: exp(-2 pi i X/W) FFT_N((-1)^n ro[n])[X mod N] with
+  // ro[n] = exp(+2 pi i k (2n+1)/W)/W (k = kx, resp. -ky), i.e. the prefactor times
   // exp(i phi0)/W * sum_n exp(i theta n), theta = 4 pi k/W + pi - 2 pi m/N, in closed form
-  std::vector<float2> nyq((size_t)nA * nPair * 2 * N);
+  std::vector<float2> nyq((size_t)nA * nPair * 2 * nwin);
   for (int a = 0; a < nA; a++)
     for (int b = 1; b <= nPair; b++) {
+      const int cn = 2 * b - 1;
       double kx, ky;
-      comp_shift(&prm, a, 2 * b, &kx, &ky);
+      comp_shift(&prm, a, cn, &kx, &ky);
       for (int dim = 0; dim < 2; dim++) {
         const double k = dim == 0 ? kx : -ky;
         const double f0 = k / W - std::floor(k / W), f1 = 2 * k / W - std::floor(2 * k / W);
         const std::complex<double> e0 = std::polar(1.0 / W, 2 * M_PI * f0);
-        for (int m = 0; m < N; m++) {
+        for (int l = 0; l < nwin; l++) {
+          const int X = (win[2 * (a * nC + cn) + dim] + l) % W, m = X % N;
           double th = 2 * M_PI * f1 + M_PI - 2 * M_PI * (double)m / N;
           th -= 2 * M_PI * std::floor(th / (2 * M_PI) + 0.5);  // (-pi, pi]
           std::complex<double> S;
@@ -183,8 +177,8 @@ int Plan::build(cudaStream_t st) {
             fn -= std::floor(fn);
             S = (1.0 - std::polar(1.0, 2 * M_PI * fn)) / (1.0 - std::polar(1.0, th));
           }
-          const std::complex<double> q = e0 * S;
-          nyq[(((size_t)a * nPair + (b - 1)) * 2 + dim) * N + m] = make_float2((float)q.real(), (float)q.imag());
+          const std::complex<double> q = std::polar(1.0, -2 * M_PI * (double)X / W) * e0 * S;
+          nyq[(((size_t)a * nPair + (b - 1)) * 2 + dim) * nwin + l] = make_float2((float)q.real(), (float)q.imag());
         }
       }
     }
@@ -196,7 +190,7 @@ int Plan::build(cudaStream_t st) {
   size_t off_damp = off_otf + al(sizeof(OtfTable));
   size_t off_mask = off_damp + al((size_t)N * N * sizeof(float));
   const size_t mask_elem = otf_measured(&prm) ? sizeof(float2) : sizeof(float);
-  size_t off_wa = off_mask + al((size_t)nA * nC * nwin * nwin * mask_elem);
+  size_t off_wa = off_mask + al((size_t)(1 + nA * nPair) * nwin * nwin * mask_elem);
   // Wiener x apo over the Hermitian half read by pass B2 (columns X <= N in whole quads),
   // then the apodization's octant table ((N + 1)^2 floats, plan build only)
   const size_t wa_elems = (size_t)(N + 4) * W, apo_elems = (size_t)(N + 1) * (N + 1);
@@ -232,15 +226,15 @@ int Plan::build(cudaStream_t st) {
   }
   FSIM_CUDA(cudaStreamSynchronize(st));
   // masks (exact double-precision OTF lookups), Wiener x apo
-  for (int a = 0; a < nA; a++)
-    for (int c = 0; c < nC; c++) {
-      double kx, ky;
-      comp_shift(&prm, a, c, &kx, &ky);
-      dim3 g(div_up(nwin, 128), nwin);
-      k_build_mask<<<g, 128, 0, st>>>(d_masks + (size_t)(a * nC + c) * nwin * nwin * (mask_elem / sizeof(float)), W,
-                                      nwin, win[2 * (a * nC + c)], win[2 * (a * nC + c) + 1], kx, ky,
-                                      fshift_host(kx, ky), d_otf, prm.use_attenuation, (c + 1) / 2);
-    }
+  for (int s = 0; s <= nA * nPair; s++) {
+    const int a = s ? (s - 1) / nPair : 0, c = s ? 2 * ((s - 1) % nPair) + 1 : 0;
+    double kx, ky;
+    comp_shift(&prm, a, c, &kx, &ky);
+    dim3 g(div_up(nwin, 128), nwin);
+    k_build_mask<<<g, 128, 0, st>>>(d_masks + (size_t)s * nwin * nwin * (mask_elem / sizeof(float)), W, nwin,
+                                    win[2 * (a * nC + c)], win[2 * (a * nC + c) + 1], kx, ky, fshift_host(kx, ky),
+                                    d_otf, prm.use_attenuation, (c + 1) / 2, s ? 1.f : 0.5f);
+  }
   {
     float* d_apo = d_wa + wa_elems;
     int rc = apo_octant_device(d_apo, N, ht.vec_cpm, ht.cutoff * prm.apo_cutoff, prm.apo_bend, st);
@@ -260,23 +254,22 @@ int Plan::build(cudaStream_t st) {
   return FSIM_OK;
 }
 
-// workspace of one dataset: I | D | G | Tw | Dy | O | On | clip max (each 256-byte aligned).
+// workspace of one dataset: I | D | G | Tw | O | On | clip max (each 256-byte aligned).
 // I holds the band-0 slot (all angles summed) and one slot per angle and band pair.
-static void ws_parts(const fsim_sim_param& p, int nwin, size_t part[8]) {
+static void ws_parts(const fsim_sim_param& p, int nwin, size_t part[7]) {
   const int N = p.w, W = 2 * N, nPair = p.nr_bands - 1;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   part[0] = al((size_t)(1 + p.nr_dirs * nPair) * nwin * N * sizeof(float2));
   part[1] = al((size_t)p.nr_dirs * nPair * N * sizeof(float2));
   part[2] = al((size_t)p.nr_dirs * nPair * nwin * sizeof(float2));
   part[3] = al((size_t)(1 + p.nr_dirs * nPair) * nwin * nwin * sizeof(float2));
-  part[4] = al((size_t)p.nr_dirs * nPair * nwin * sizeof(float2));
-  part[5] = al((size_t)W * N * sizeof(float2));
-  part[6] = al((size_t)W * sizeof(float2));
-  part[7] = 256;
+  part[4] = al((size_t)W * N * sizeof(float2));
+  part[5] = al((size_t)W * sizeof(float2));
+  part[6] = 256;
 }
 
 size_t Plan::workspace_bytes() const {
-  size_t part[8];
+  size_t part[7];
   ws_parts(prm, nwin, part);
   size_t sum = 0;
   for (size_t v : part) sum += v;
@@ -307,17 +300,16 @@ void Plan::fill_job(JobDesc& j, const void* raw, float* out, float* wf, float* f
   j.masks = d_masks;
   j.wa = d_wa;
   j.nyq = d_nyq;
-  size_t part[8];
+  size_t part[7];
   ws_parts(prm, nwin, part);
   char* w = ws;
   j.I = (float2*)w;
   j.D = (float2*)(w += part[0]);
   j.G = (float2*)(w += part[1]);
   j.Tw = (float2*)(w += part[2]);
-  j.Dy = (float2*)(w += part[3]);
-  j.O = (float2*)(w += part[4]);
-  j.On = (float2*)(w += part[5]);
-  j.clip_max = (float*)(w += part[6]);
+  j.O = (float2*)(w += part[3]);
+  j.On = (float2*)(w += part[4]);
+  j.clip_max = (float*)(w += part[5]);
 }
 
 // ---- autotuned variants ------------------------------------------------------------------------

@@ -19,16 +19,17 @@ struct JobDesc {
   const float2* coef;   // [a][c][p] separation coefficients
   const float2* ramps;  // [a][c] {x ramp[W], y ramp[W]}  (offline) / {x ramp[N], y ramp[N]} (live)
   const int* win;       // [a][c] {Xs, Ys} window origins (offline) / {xInt, yInt} paste offsets (live)
-  const float* masks;   // [a][c] OTF masks (offline; float2 when cmask) / N*N conj-OTF vector (live)
+  const float* masks;   // OTF masks [band 0 (halved), neg of (a, b)][nWin column][nWin row] (offline; float2 when
+                        // cmask) / N*N conj-OTF vector (live)
   const float* wa;      // Wiener x apodization, quad layout [X/4][Y][X%4]
-  const float2* nyq;    // offline: [a][b-1][x, y][N] FFT_N((-1)^n ro_pos[n]) of the pos component's x and y
-                        // odd-sample ramps (the Nyquist response, see pass A)
+  const float2* nyq;    // offline: [a][b-1][x over the neg window's columns, y over its rows][nWin]: response of
+                        // the neg component's odd-sample shift to the Nyquist bin (pass A)
   float2* I;            // workspace: row-transformed windows [band 0, neg of (a, b)][nWin/4][N][4] (offline);
                         // live: [a][c] N*N row transforms
-  float2* D;            // workspace: [a][b-1][N] Nyquist term d of every row's neg component (pass A)
-  float2* G;            // workspace: [a][b-1][nWin] column transform of D with the pos y shift (pass G)
-  float2* Tw;           // workspace: column-transformed windows [band 0, neg of (a, b)][nWin/4][nWin][4] (pass B1)
-  float2* Dy;           // workspace: [a][b-1][nWin] Nyquist term d' of every neg window column (pass B1)
+  float2* D;            // workspace: [a][b-1][N] Nyquist bin of every row's neg component (pass A)
+  float2* G;            // workspace: [a][b-1][nWin] column transform of D (pass G, complex masks only)
+  float2* Tw;           // workspace: masked column-transformed windows [band 0, neg of (a, b)][nWin column]
+                        // [nWin row] (pass B1)
   float2* O;            // workspace: offline: W x N, columns 0..N-1 of the Hermitian half after pass B2
                         // (row-major, stride N); live: W*W after the column pass
   float2* On;           // workspace (offline): column N of the Hermitian half, W entries

@@ -27,9 +27,8 @@ const char* last_error() { return g_errbuf; }
 
 // Test hook: the n-th next device allocation of the library fails (fsim_debug_fail_alloc).
 static std::atomic<int> g_fail_alloc{0};
-// Pass B2's bulk-copy staging on (fsim_debug_b2_staging)
+// The setting of fsim_debug_b2_staging, which no longer selects anything
 static std::atomic<int> g_b2_staging{1};
-bool b2_staging_enabled() { return g_b2_staging.load(std::memory_order_relaxed) != 0; }
 
 cudaError_t dev_alloc(void** p, size_t bytes) {
   int n = g_fail_alloc.load();

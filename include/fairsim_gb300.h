@@ -208,12 +208,11 @@ int fsim_plan_info(const fsim_plan* plan, int* w, int* path, int* input_type);
  * plans. n_floats must hold 2w * ncols values; *ncols receives ncols. Synchronises the device. */
 /* Bits set on the device since the last clear by kernels that detected a failure instead of
  * hanging or faulting (FSIM_STATUS_*; 0 when none): read after the work has finished.
- * detail (nullable, 3 ints) receives a description of the first event (kernel-specific:
- * pass B2 records (block x) | (stage << 12) | (stages << 18) | (depth << 24), then the two
- * 32-bit halves of the barrier word it waited on). Synchronises the device; clear != 0
- * resets the words. */
-#define FSIM_STATUS_BULK_WAIT 1    /* pass B2: a staged bulk copy was not seen complete in time */
-#define FSIM_STATUS_STAGE_LAYOUT 2 /* pass B2: a stage would span more than two column quads */
+ * detail (nullable, 3 ints) receives a description of the first event (kernel-specific).
+ * Synchronises the device; clear != 0 resets the words. The current kernels wait on nothing
+ * but their own block's barriers and set no bit; the values stay reserved. */
+#define FSIM_STATUS_BULK_WAIT 1    /* a staged bulk copy was not seen complete in time */
+#define FSIM_STATUS_STAGE_LAYOUT 2 /* a stage would span more than two column quads */
 int fsim_device_status(int* bits, int* detail, int clear);
 int fsim_plan_filter_table(const fsim_plan* plan, float* host_out, size_t n_floats, int* ncols);
 /* Output scaling of an offline plan's reconstruction, SimParam.CLIPSCALE
@@ -314,10 +313,9 @@ int fsim_corr_grid_noalloc(const void* b0, const void* b1, int n, const double* 
  * The nth next device allocation made by the library (nth >= 1) fails as out of memory;
  * 0 disarms. Lets tests drive every FSIM_EOOM path without exhausting a shared GPU. */
 int fsim_debug_fail_alloc(int nth);
-/* Pass B2 of the fused offline path stages its inputs into shared memory with bulk copies
- * where they fit (on = 1, the default) or reads them with plain loads (on = 0); both give the
- * same bits. *prev (nullable) receives the previous setting. Lets tests and benchmarks compare
- * the two. */
+/* Kept for programs that switch it: pass B2 of the fused offline path had a staged and a
+ * plain-load form with the same bits and now has one. *prev (nullable) receives the previous
+ * setting; the results do not depend on it. */
 int fsim_debug_b2_staging(int on, int* prev);
 
 /* ---- served form: continuous batching over channels (replaces ReconstructionRunner) --- */
