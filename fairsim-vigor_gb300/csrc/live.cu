@@ -8,16 +8,33 @@
 //
 // The fractional shift FFT_N(ramp * iFFT_N(.)) is separable, but the OTF product sits
 // between the forward transforms and the shift, so four passes are used:
-//   LA rows    (per dataset x raw row):     damp, widefield, band mix, FFT_N along x
-//   LB columns (per dataset x 4 columns):   FFT_N along y, x conj(OTF), y half of the shift
-//   LC rows    (per dataset x output row):  x half of the shift, paste at the integer
-//                                           offsets, sum, x Wiener*apo, iFFT_W along x
-//   LD columns (per dataset x 8 columns):   iFFT_W along y, real part, 1/W^2
+//   LA rows    (per dataset x raw row pair):  damp, widefield, band mix, FFT_N along x
+//   LB columns (per dataset x 4 columns):     FFT_N along y, x conj(OTF), y half of the shift
+//   LC rows    (per dataset x output row pair): x half of the shift, paste at the integer
+//                                             offsets, sum, x Wiener*apo, iFFT_W along x
+//   LD columns (per dataset x columns):       complex-to-real inverse along y, 1/W^2
+// Three symmetries leave 4 of the 9 components of a 3 x 3 stack, and half of the output grid:
+//  * band 0 of every angle has the same OTF and no shift: the angles are summed before LA's
+//    transform;
+//  * the neg component of a band pair is the conjugate of the pos one in real space, and the
+//    fast shift's two ramps are conjugates up to a whole bin: with V the shifted pos spectrum,
+//    fx = kx - floor(kx), dx = (fx != 0) and likewise along y,
+//      V_neg[m, n] = conj V[dx - m, dy - n]   (indices modulo N),
+//    pasted at -floor(kx) - dx. So V sits at X = floor(kx) + p, p in [-N/2, N/2 - 1], and its
+//    conjugate mirror image at X = -(floor(kx) + p), p in [dx - N/2 + 1, dx + N/2];
+//  * the image is real: only H(X, Y) = (F(X, Y) + conj F(-X, -Y)) / 2 matters, to which V[p]
+//    contributes at +-(floor(k) + p) with weight 1, or 1/2 for the bins on the edge of the two
+//    ranges, and only the rows Y = 0..N of H are formed (LD completes each column by symmetry).
+// The OTF also zeroes every column beyond its support: only a window of columns leaves LA.
+// Rows (LA, LC) and columns (LB, LD) are transformed two at a time (fft_pair.cuh). Bound by the
+// shared-memory pipe and instruction issue of 11.6k transforms of length N per 512^2 3x3 stack (26k
+// with every component and the full grid): 64 stacks in 1116 us on GB300, 2382 us before; one
+// stack 66.7 us, 109 before.
 #include <cmath>
 #include <vector>
 
 #include "common.cuh"
-#include "fft_line.cuh"
+#include "fft_pair.cuh"
 #include "filters.cuh"
 #include "otf.cuh"
 #include "recon.cuh"
@@ -32,231 +49,369 @@ int plan_window(const fsim_sim_param* p, double R, int* nwin);
 template <int N>
 struct LCfg {
   static constexpr int W = 2 * N;
-  static constexpr int EN = (N % 3 == 0) ? 12 : 16;
-  static constexpr int TN = N / EN;                            // threads per N-line
-  static constexpr int GA = TN >= 128 ? 1 : 128 / TN;          // rows per block, pass LA
-  static constexpr int CBL = 4;                                // columns per block, pass LB
-  static constexpr int EW = (N % 3 == 0) ? 24 : 16;
-  static constexpr int TW = W / EW;                            // threads per W-line
-  static constexpr int CD = (N >= 2048) ? 2 : (N >= 1024 ? 4 : 8);  // columns per block, pass LD
+  static constexpr int E = (N % 3 == 0) ? 12 : 8;
+  static constexpr int T = N / E;                   // threads per line pair
+  static constexpr int G = T >= 64 ? 1 : 64 / T;    // row pairs per block, passes LA and LC
+  static constexpr int CP = 2;                      // column pairs per block, pass LB
+  static constexpr int CD = N >= 2048 ? 2 : 4;      // column pairs per block, pass LD
+  static constexpr int R = E <= 8 ? 80 : 128;       // registers per thread
+  static constexpr int blocks(int threads) {
+    const int n = threads < 32 ? 32 : threads, b = 65536 / (n * R);
+    return b < 1 ? 1 : (b > 32 ? 32 : b);
+  }
+  static constexpr int XS = pair_elems(N, 1);       // exchange buffer of one pair
 };
-
-// Register budget of about 80 per thread for the column and shift passes (they otherwise keep
-// 120-130 and run at 16 warps per SM).
-__host__ __device__ constexpr int live_min_blocks(int threads) {
-  return 65536 / (threads * 80) > 0 ? 65536 / (threads * 80) : 1;
-}
-
-// pasteFreq's source index for output index o (as in vec_ops.cu)
-__device__ __forceinline__ int paste_source(int o, int off, int ni, int no) {
-  int p1 = ((o - off) % no + no) % no;
-  int p2 = ((o - off - no / 2) % no + no) % no;
-  int best = -1;
-  if (p1 < ni / 2) best = p1;
-  if (p2 >= ni / 2 && p2 < ni && p2 > best) best = p2;
-  return best;
+// window column of spectrum column m (nWin columns from Xs, modulo N), or beyond nWin
+template <int N>
+__device__ __forceinline__ int live_col(int m, int Xs) {
+  const int x = m - Xs;
+  return x < 0 ? x + N : x;
 }
 
 // ---- LA -----------------------------------------------------------------------------------
+// blockIdx.y < nA: the pos components of that angle; blockIdx.y == nA: band 0 of all angles, and
+// the widefield.
 template <int N>
-__global__ void __launch_bounds__(LCfg<N>::GA* LCfg<N>::TN) k_live_a(const JobDesc* __restrict__ jobs) {
+__global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N>::G* LCfg<N>::T))
+    k_live_a(const JobDesc* __restrict__ jobs) {
   using P = LCfg<N>;
-  constexpr int T = P::TN, G = P::GA, E = P::EN;
-  const JobDesc& J = jobs[blockIdx.y];
+  constexpr int T = P::T, G = P::G, E = P::E;
+  const JobDesc& J = jobs[blockIdx.z];
   const int g = threadIdx.x / T, t = threadIdx.x % T;
-  const int y = blockIdx.x * G + g;
-  __shared__ float2 sm[G * smem_line_elems(N, 1)];
+  const int y = 2 * (blockIdx.x * G + g), a = blockIdx.y;
+  extern __shared__ ulonglong2 smp[];
+  ulonglong2* s = smp + g * P::XS;
   const float2* tw = g_stw + stw_offset(N, E);  // stage twiddles through L1
-  float2* s = sm + g * smem_line_elems(N, 1);
   const size_t frame = (size_t)N * N, row = (size_t)y * N;
-  const float* rawf = (const float*)J.raw;
-  const uint16_t* rawu = (const uint16_t*)J.raw;
-  const int nA = J.nA, nP = J.nP, nC = J.nC;
-  // setFrom16bitPixels + times(dampBorder) of the row of frame f at this thread's elements
-  // t + i*T; frames outer and elements inner, so that a row's E loads are in flight at once
-  auto px_row = [&](int f, float (&v)[E]) {
+  const int nA = J.nA, nP = J.nP, nC = J.nC, nPair = (nC - 1) / 2, nWin = J.nWin, Xs = J.win[0];
+  if (a > nA) return;  // uniform per block
+  // setFrom16bitPixels + times(dampBorder) of both rows of frame f at this thread's elements
+  // t + i*T; frames outer and elements inner, so that the rows' loads are in flight at once
+  auto px_rows = [&](int f, f32x2 (&v)[E]) {
     const size_t at = (size_t)f * frame + row + t;
     if (J.input_u16) {
+      const uint16_t* r = (const uint16_t*)J.raw + at;
 #pragma unroll
-      for (int i = 0; i < E; i++) v[i] = (float)__ldg(&rawu[at + i * T]);
+      for (int i = 0; i < E; i++) v[i] = p_pack((float)__ldg(r + i * T), (float)__ldg(r + N + i * T));
     } else {
+      const float* r = (const float*)J.raw + at;
 #pragma unroll
-      for (int i = 0; i < E; i++) v[i] = __ldg(&rawf[at + i * T]);
+      for (int i = 0; i < E; i++) v[i] = p_pack(__ldg(r + i * T), __ldg(r + N + i * T));
     }
     if (J.damp) {
+      const float* d = J.damp + row + t;
 #pragma unroll
-      for (int i = 0; i < E; i++) v[i] = __fmul_rn(v[i], __ldg(&J.damp[row + t + i * T]));
+      for (int i = 0; i < E; i++) v[i] = p_mul(v[i], p_pack(__ldg(d + i * T), __ldg(d + N + i * T)));
     }
   };
-  if (J.widefield) {
-    const float sc = 1.f / (float)(nA * nP);
-    float wf[E];
+  // both rows' value of the window columns, to the quad layout [xl/4][y][xl%4]
+  cpair x[E];  // element t + i*T of both rows, in registers through the transform
+  auto put = [&](int slot) {
+    float2* I = J.I + (size_t)slot * nWin * N;
 #pragma unroll
-    for (int i = 0; i < E; i++) wf[i] = 0.f;
+    for (int i = 0; i < E; i++) {
+      const int xl = live_col<N>(t + i * T, Xs);
+      if (xl < nWin) {
+        float2 r0, r1;
+        cp_split(x[i], r0, r1);
+        float2* o = I + ((size_t)(xl >> 2) * N + y) * 4 + (xl & 3);
+        o[0] = r0;
+        o[4] = r1;
+      }
+    }
+  };
+  if (a == nA) {
+    f32x2 wf[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+      x[i] = cp_zero();
+      wf[i] = 0ull;
+    }
 #pragma unroll 1
     for (int f = 0; f < nA * nP; f++) {
-      float v[E];
-      px_row(f, v);
+      f32x2 v[E];
+      px_rows(f, v);
+      const wpair m = w_dup(__ldg(J.coef + (f / nP) * nC * nP + f % nP));
 #pragma unroll
-      for (int i = 0; i < E; i++) wf[i] = __fadd_rn(wf[i], v[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < E; i++) J.widefield[row + t + i * T] = __fmul_rn(wf[i], sc);
-  }
-  for (int a = 0; a < nA; a++)
-    for (int c = 0; c < nC; c++) {
-      const float2* coef = J.coef + (a * nC + c) * nP;
-      float2 xv[E];  // element t + i*T of the line, in registers through the transform
-#pragma unroll
-      for (int i = 0; i < E; i++) xv[i] = make_float2(0.f, 0.f);
-#pragma unroll 1
-      for (int p = 0; p < nP; p++) {
-        float v[E];
-        px_row(a * nP + p, v);
-        const float2 m = coef[p];
-#pragma unroll
-        for (int i = 0; i < E; i++) {
-          xv[i].x += m.x * v[i];
-          xv[i].y += m.y * v[i];
-        }
+      for (int i = 0; i < E; i++) {
+        wf[i] = p_add(wf[i], v[i]);
+        x[i] = cpair{p_fma(m.x, v[i], x[i].re), p_fma(m.y, v[i], x[i].im)};
       }
-      line_fft_reg<N, T, 1, false>(xv, s, 0, t, tw);
-      float2* X = J.I + (size_t)(a * nC + c) * frame + row;
-#pragma unroll
-      for (int i = 0; i < E; i++) X[t + i * T] = xv[i];
     }
+    if (J.widefield) {
+      const f32x2 sc = p_dup(1.f / (float)(nA * nP));
+#pragma unroll
+      for (int i = 0; i < E; i++) {
+        const float2 w = p_unpack(p_mul(wf[i], sc));
+        J.widefield[row + t + i * T] = w.x;
+        J.widefield[row + N + t + i * T] = w.y;
+      }
+    }
+    line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
+    put(0);
+    return;
+  }
+  for (int b = 1; b <= nPair; b++) {
+    const float2* coef = J.coef + (a * nC + 2 * b) * nP;
+#pragma unroll
+    for (int i = 0; i < E; i++) x[i] = cp_zero();
+#pragma unroll 1
+    for (int p = 0; p < nP; p++) {
+      f32x2 v[E];
+      px_rows(a * nP + p, v);
+      const wpair m = w_dup(__ldg(coef + p));
+#pragma unroll
+      for (int i = 0; i < E; i++) x[i] = cpair{p_fma(m.x, v[i], x[i].re), p_fma(m.y, v[i], x[i].im)};
+    }
+    line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
+    put(1 + a * nPair + (b - 1));
+  }
 }
 
 // ---- LB -----------------------------------------------------------------------------------
 template <int N>
-__global__ void __launch_bounds__(LCfg<N>::CBL* LCfg<N>::TN, live_min_blocks(LCfg<N>::CBL* LCfg<N>::TN))
+__global__ void __launch_bounds__(LCfg<N>::CP* LCfg<N>::T, LCfg<N>::blocks(LCfg<N>::CP* LCfg<N>::T))
     k_live_b(const JobDesc* __restrict__ jobs) {
   using P = LCfg<N>;
-  constexpr int T = P::TN, C = P::CBL, E = P::EN;
-  const JobDesc& J = jobs[blockIdx.y];
+  constexpr int T = P::T, C = P::CP, E = P::E;
+  const JobDesc& J = jobs[blockIdx.z];
   const int lt = threadIdx.x, lane = lt % C, t = lt / C;
-  const int x = blockIdx.x * C + lane;
-  __shared__ float2 s[smem_line_elems(N, C)];
-  const float2* tw = g_stw + stw_offset(N, E);  // stage twiddles through L1
-  const size_t frame = (size_t)N * N;
-  for (int a = 0; a < J.nA; a++)
-    for (int c = 0; c < J.nC; c++) {
-      float2* X = J.I + (size_t)(a * J.nC + c) * frame;
-      float2 v[E];  // element t + i*T of this lane's column, in registers through the transforms
+  const int nPair = (J.nC - 1) / 2, nWin = J.nWin, slot = blockIdx.y;
+  if (slot > J.nA * nPair || (int)blockIdx.x * 2 * C >= nWin) return;  // uniform per block
+  const int xl = blockIdx.x * 2 * C + 2 * lane;  // and xl + 1: nWin is a multiple of 4
+  extern __shared__ ulonglong2 smp[];
+  const float2* tw = g_stw + stw_offset(N, E);
+  // rows two float4 apart; the columns are this block's alone and are transformed in place
+  float4* I = reinterpret_cast<float4*>(J.I + (size_t)slot * nWin * N + ((size_t)(xl >> 2) * N) * 4 + (xl & 3));
+  cpair x[E];  // element t + i*T of both columns, in registers through the transforms
 #pragma unroll
-      for (int i = 0; i < E; i++) v[i] = X[(size_t)(t + i * T) * N + x];
-      line_fft_reg<N, T, C, false>(v, s, lane, t, tw);
-      // times conj(OTF): the OTF vector is real (estimate), conj(OTF)*v = (v.re*o, v.im*o)
+  for (int i = 0; i < E; i++) {
+    const float4 v = I[(size_t)(t + i * T) * 2];
+    x[i] = cpair{p_pack(v.x, v.z), p_pack(v.y, v.w)};
+  }
+  line_fft_pair<N, T, C, false>(x, smp, lane, t, tw);
+  // times conj(OTF): the OTF vector is real (estimate); band 0 carries its weight 1/2
+  const float* o = J.masks + (size_t)xl * N + t;
+  const float h = slot == 0 ? 0.5f : 1.f;
 #pragma unroll
-      for (int i = 0; i < E; i++) {
-        const float o = __ldg(&J.masks[(size_t)(t + i * T) * N + x]);
-        v[i] = make_float2(__fmul_rn(v[i].x, o), __fmul_rn(v[i].y, o));
-      }
-      if (c > 0) {
-        line_fft_reg<N, T, C, true>(v, s, lane, t, tw);
-        const float2* ry = J.ramps + (size_t)(a * J.nC + c) * 2 * N + N;
+  for (int i = 0; i < E; i++) {
+    const f32x2 f = p_pack(h * __ldg(o + i * T), h * __ldg(o + N + i * T));
+    x[i] = cpair{p_mul(x[i].re, f), p_mul(x[i].im, f)};
+  }
+  if (slot > 0) {
+    line_fft_pair<N, T, C, true>(x, smp, lane, t, tw);
+    const float2* ry = J.ramps + (size_t)(slot - 1) * 2 * N + N;
 #pragma unroll
-        for (int i = 0; i < E; i++) v[i] = cmul(v[i], __ldg(&ry[t + i * T]));
-        line_fft_reg<N, T, C, false>(v, s, lane, t, tw);
-      }
+    for (int i = 0; i < E; i++) x[i] = cmul(x[i], w_dup(__ldg(ry + t + i * T)));
+    line_fft_pair<N, T, C, false>(x, smp, lane, t, tw);
+  }
 #pragma unroll
-      for (int i = 0; i < E; i++) X[(size_t)(t + i * T) * N + x] = v[i];
-    }
+  for (int i = 0; i < E; i++) {
+    float2 r0, r1;
+    cp_split(x[i], r0, r1);
+    I[(size_t)(t + i * T) * 2] = make_float4(r0.x, r0.y, r1.x, r1.y);
+  }
 }
 
 // ---- LC -----------------------------------------------------------------------------------
+// One row pair (Y, Y + 1) of H per group of T threads, Y even, Y <= N. The rows of a slot that
+// land on them directly (row Y - floor(ky)) or mirrored (row -Y - floor(ky)) are transformed as
+// a pair and added to the rows' sums in shared memory; then x Wiener*apo, and iFFT_W along x as
+// two N-point inverse transforms (even and odd samples).
 template <int N>
-__global__ void __launch_bounds__(LCfg<N>::TW, live_min_blocks(LCfg<N>::TW)) k_live_c(const JobDesc* __restrict__ jobs) {
+struct LCPass {
   using P = LCfg<N>;
-  constexpr int W = P::W, TW = P::TW, EW = P::EW, EN = N / TW;
+  static constexpr int NT = P::G * P::T;
+  static constexpr int GS = P::XS + 2 * N;  // exchange buffer and the sums of a row pair
+  static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)P::G * GS;
+};
+template <int N>
+__global__ void __launch_bounds__(LCPass<N>::NT, LCfg<N>::blocks(LCPass<N>::NT))
+    k_live_c(const JobDesc* __restrict__ jobs) {
+  using P = LCfg<N>;
+  constexpr int W = P::W, T = P::T, E = P::E, G = P::G;
   const JobDesc& J = jobs[blockIdx.y];
-  const int Y = blockIdx.x, t = threadIdx.x;
-  // Stage twiddles are read through L1 (g_stw), as in the offline passes: per-block copies in
-  // shared memory held the pass to 16 warps per SM. Row values outside the transforms (the
-  // paste read-out, the sum) use the unpadded index: a half-warp's 16 consecutive float2 then
-  // fall into distinct bank pairs from any starting element.
-  __shared__ float2 acc[smem_line_elems(W, 1)];
-  __shared__ float2 s[smem_line_elems(N, 1)];
-  const float2* twN = g_stw + stw_offset(N, EN);
-  const float2* twW = g_stw + stw_offset(W, EW);
+  const int g = threadIdx.x / T, t = threadIdx.x % T;
+  const int Y0 = 2 * (blockIdx.x * G + g);  // rows Y0 and Y0 + 1; stored up to row N
+  extern __shared__ ulonglong2 smp[];
+  ulonglong2* s = smp + g * LCPass<N>::GS;
+  ulonglong2* acc = s + P::XS;  // (re, im) of both rows, W columns
+  const float2* tw = g_stw + stw_offset(N, E);
+  const float2* twW = g_tw + tw_offset(W);
+  const int nPair = (J.nC - 1) / 2, nWin = J.nWin, Xs = J.win[0], nS = 1 + J.nA * nPair;
+  const float* wa = J.wa;
+  auto wrap = [](int v) { return v < 0 ? v + W : (v >= W ? v - W : v); };
 #pragma unroll
-  for (int i = 0; i < EW; i++) acc[t + i * TW] = make_float2(0.f, 0.f);
-  const size_t frame = (size_t)N * N;
-  for (int a = 0; a < J.nA; a++)
-    for (int c = 0; c < J.nC; c++) {
-      const int xInt = J.win[2 * (a * J.nC + c)], yInt = J.win[2 * (a * J.nC + c) + 1];
-      const int ys = paste_source(Y, yInt, N, W);
-      if (ys < 0) continue;  // uniform per block
-      const float2* X = J.I + (size_t)(a * J.nC + c) * frame + (size_t)ys * N;
-      float2 v[EN];  // element t + i*TW of the row, in registers through the transforms
+  for (int i = 0; i < 2 * E; i++) acc[t + i * T] = make_ulonglong2(0ull, 0ull);
+  // One contribution: rows q0 and q0 + d of the slot (relative to its origin; d = -1 mirrored).
+  // u[h] are the weights of the direct and the mirrored range for row h.
+  cpair x[E];
+  auto load_row = [&](const float2* I, int q, bool on, float2 (&v)[E]) {
+    const int ys = q < 0 ? q + N : (q >= N ? q - N : q);
 #pragma unroll
-      for (int i = 0; i < EN; i++) v[i] = X[t + i * TW];
-      __syncthreads();  // the previous paste has read s
-      if (c > 0) {
-        line_fft_reg<N, TW, 1, true>(v, s, 0, t, twN);
-        const float2* rx = J.ramps + (size_t)(a * J.nC + c) * 2 * N;
-#pragma unroll
-        for (int i = 0; i < EN; i++) v[i] = cmul(v[i], __ldg(&rx[t + i * TW]));
-        line_fft_reg<N, TW, 1, false>(v, s, 0, t, twN);
-      }
-#pragma unroll
-      for (int i = 0; i < EN; i++) s[t + i * TW] = v[i];
-      __syncthreads();
-      // pasteFreq at (xInt, yInt) and fullResult.add
-#pragma unroll
-      for (int i = 0; i < EW; i++) {
-        const int Xo = t + i * TW;
-        const int xs = paste_source(Xo, xInt, N, W);
-        if (xs >= 0) {
-          float2& o = acc[Xo];
-          const float2 v = s[xs];
-          o = make_float2(__fadd_rn(o.x, v.x), __fadd_rn(o.y, v.y));
-        }
-      }
-      __syncthreads();
+    for (int i = 0; i < E; i++) {
+      const int xl = live_col<N>(t + i * T, Xs);
+      v[i] = (on && xl < nWin) ? __ldg(I + ((size_t)(xl >> 2) * N + ys) * 4 + (xl & 3)) : make_float2(0.f, 0.f);
     }
-  const float* wa = J.wa + (size_t)Y * W;
-  float2 u[EW];
+  };
+  for (int sl = 0; sl < nS; sl++) {
+    const float2* I = J.I + (size_t)sl * nWin * N;
+    const int* w = J.win + 4 * sl;  // slot 0: (Xs, 0, -, -); pairs: floor(kx), floor(-ky), dx, dy
+    const int xi = sl ? w[0] : 0, yi = sl ? w[1] : 0, dx = sl ? w[2] : 0, dy = sl ? w[3] : 0;
+    for (int mir = 0; mir < 2; mir++) {
+      // Rows of the slot, relative to its origin: in the pos range [-N/2, N/2 - 1], in the neg
+      // range [dy - N/2 + 1, dy + N/2] (band 0: the pos range only, its mirror image included).
+      int q[2];
+      float wp[2], wn[2];  // weights of an element inside the pos / the neg x range
+      bool any = false;
 #pragma unroll
-  for (int i = 0; i < EW; i++) {
-    const int k = t + i * TW;
-    const float f = __ldg(&wa[k]);
-    const float2 o = acc[k];
-    u[i] = make_float2(o.x * f, o.y * f);
+      for (int h = 0; h < 2; h++) {
+        q[h] = (mir ? -(Y0 + h) : Y0 + h) - yi;
+        if (q[h] < -N) q[h] += W;  // floor(k) shifts reach beyond the grid's half
+        else if (q[h] >= N) q[h] -= W;
+        const bool in_p = q[h] >= -N / 2 && q[h] <= N / 2 - 1;
+        const bool in_n = q[h] >= dy - N / 2 + 1 && q[h] <= dy + N / 2;
+        wp[h] = sl ? (in_p ? 0.5f : 0.f) : (in_p ? 1.f : 0.f);
+        wn[h] = sl && in_n ? 0.5f : 0.f;
+        any = any || in_p || (sl && in_n);
+      }
+      any = __syncthreads_or(any);  // the same for every row pair of the block; orders the sums, too
+      if (!any) continue;
+      {
+        float2 r0[E], r1[E];
+        load_row(I, q[0], wp[0] + wn[0] > 0.f, r0);
+        load_row(I, q[1], wp[1] + wn[1] > 0.f, r1);
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = cp_make(r0[i], r1[i]);
+      }
+      if (sl) {
+        line_fft_pair<N, T, 1, true>(x, s, 0, t, tw);
+        const float2* rx = J.ramps + (size_t)(sl - 1) * 2 * N;
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = cmul(x[i], w_dup(__ldg(rx + t + i * T)));
+        line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
+      }
+      // v at p = px; sp, sn: inside the pos / the neg range along x
+      auto add = [&](int px, bool sp, bool sn, cpair v) {
+        int X = xi + px;
+        if (mir) X = -X;
+        X = wrap(wrap(X));
+        float u[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float fp = 1.f, fn = 1.f;
+          if (X == N || Y0 == N) {
+            // The Nyquist column and row are their own mirror images, but Wiener and apodization
+            // differ between the coordinates -N and +N: each part is weighted here, at its own
+            // position (the pos range's at floor(k) + p, the neg range's at the mirrored one).
+            const float f0 = __ldg(wa + (size_t)(Y0 + h) * W + X);
+            const float f1 = __ldg(wa + (size_t)wrap(-(Y0 + h)) * W + wrap(-X));
+            fp = mir ? f1 : f0;
+            fn = mir ? f0 : f1;
+          }
+          u[h] = (sp ? wp[h] * fp : 0.f) + (sn ? wn[h] * fn : 0.f);
+        }
+        const f32x2 f = p_pack(u[0], u[1]);
+        ulonglong2 o = acc[X];
+        o.x = p_fma(v.re, f, o.x);
+        o.y = p_fma(v.im, mir ? p_neg(f) : f, o.y);
+        acc[X] = o;
+      };
+      // element m at p = m~ (signed), and, for the bins on the edge, at m~ + N in the neg range
+      // (no two elements of a contribution meet)
+#pragma unroll
+      for (int i = 0; i < E; i++) {
+        const int m = t + i * T, px = m < N / 2 ? m : m - N;
+        const bool in_n = px >= dx - N / 2 + 1;
+        add(px, true, in_n, x[i]);
+        if (sl && !in_n) add(px + N, false, true, x[i]);
+      }
+    }
   }
-  __syncthreads();  // acc is read: it becomes the transform's scratch
-  line_fft_reg<W, TW, 1, true>(u, acc, 0, t, twW);
-  float2* O = J.O + (size_t)Y * W;
+  __syncthreads();
+  // x Wiener*apo, then iFFT_W: out[2n] = iFFT_N(A[k] + A[k+N]), out[2n+1] = iFFT_N((A[k] - A[k+N]) e^(i pi k/N))
+  cpair z[E];
+  const int Y1 = Y0 + 1 < W ? Y0 + 1 : 0;
 #pragma unroll
-  for (int i = 0; i < EW; i++) O[t + i * TW] = u[i];
+  for (int i = 0; i < E; i++) {
+    const int k = t + i * T;
+    const ulonglong2 a = acc[k], b = acc[k + N];
+    f32x2 f0 = p_dup(1.f), f1 = p_dup(1.f);
+    if (Y0 != N) {
+      f0 = p_pack(__ldg(wa + (size_t)Y0 * W + k), __ldg(wa + (size_t)Y1 * W + k));
+      if (k != 0) f1 = p_pack(__ldg(wa + (size_t)Y0 * W + k + N), __ldg(wa + (size_t)Y1 * W + k + N));
+    }
+    const cpair u0 = cpair{p_mul(a.x, f0), p_mul(a.y, f0)}, u1 = cpair{p_mul(b.x, f1), p_mul(b.y, f1)};
+    x[i] = cadd(u0, u1);
+    z[i] = cmulj(csub(u0, u1), w_dup(__ldg(twW + k)));
+  }
+  // the odd samples wait in the sums' place (each thread its own entries)
+#pragma unroll
+  for (int i = 0; i < E; i++) acc[t + i * T] = make_ulonglong2(z[i].re, z[i].im);
+  line_fft_pair<N, T, 1, true>(x, s, 0, t, tw);
+#pragma unroll
+  for (int i = 0; i < E; i++) {
+    const ulonglong2 u = acc[t + i * T];
+    z[i] = cpair{u.x, u.y};
+    acc[t + i * T] = make_ulonglong2(x[i].re, x[i].im);
+  }
+  line_fft_pair<N, T, 1, true>(z, s, 0, t, tw);
+  // both samples of a column pair together: 16 bytes per thread and row
+#pragma unroll
+  for (int i = 0; i < E; i++) {
+    const ulonglong2 u = acc[t + i * T];
+    float2 e0, e1, o0, o1;
+    cp_split(cpair{u.x, u.y}, e0, e1);
+    cp_split(z[i], o0, o1);
+    float4* O = reinterpret_cast<float4*>(J.O + (size_t)Y0 * W) + t + i * T;
+    if (Y0 <= N) O[0] = make_float4(e0.x, e0.y, o0.x, o0.y);
+    if (Y0 < N) O[W / 2] = make_float4(e1.x, e1.y, o1.x, o1.y);
+  }
 }
 
 // ---- LD -----------------------------------------------------------------------------------
+// Column x of the image is out[y] = sum_Y h[Y] exp(+2 pi i y Y/W) / W^2 with h[W-Y] = conj h[Y]:
+// Z[k] = (h[k] + conj h[N-k]) + i exp(+2 pi i k/W) (h[k] - conj h[N-k]) gives
+// iFFT_N(Z)[n] = out[2n] + i out[2n+1].
 template <int N>
-__global__ void __launch_bounds__(LCfg<N>::CD* LCfg<N>::TW) k_live_d(const JobDesc* __restrict__ jobs) {
+__global__ void __launch_bounds__(LCfg<N>::CD* LCfg<N>::T, LCfg<N>::blocks(LCfg<N>::CD* LCfg<N>::T))
+    k_live_d(const JobDesc* __restrict__ jobs) {
   using P = LCfg<N>;
-  constexpr int W = P::W, TW = P::TW, EW = P::EW, C = P::CD;
+  constexpr int W = P::W, T = P::T, E = P::E, C = P::CD;
   const JobDesc& J = jobs[blockIdx.y];
   const int lt = threadIdx.x, lane = lt % C, t = lt / C;
-  const int X = blockIdx.x * C + lane;
-  extern __shared__ float2 s[];
-  const float2* tw = g_stw + stw_offset(W, EW);  // stage twiddles through L1
-  float2 v[EW];  // element t + i*TW of the column, in registers through the transform
+  const int X = 2 * (blockIdx.x * C + lane);
+  extern __shared__ ulonglong2 smp[];
+  const float2* tw = g_stw + stw_offset(N, E);
+  const float2* twW = g_tw + tw_offset(W);
+  const float4* O = reinterpret_cast<const float4*>(J.O) + X / 2;  // rows W/2 float4 apart
+  cpair v[E];  // element t + i*T of Z, in registers through the transform
 #pragma unroll
-  for (int i = 0; i < EW; i++) v[i] = J.O[(size_t)(t + i * TW) * W + X];
-  line_fft_reg<W, TW, C, true>(v, s, lane, t, tw);
-  const float scale = 1.f / ((float)W * (float)W);
+  for (int i = 0; i < E; i++) {
+    const int k = t + i * T;
+    const float4 a = O[(size_t)k * (W / 2)], b = O[(size_t)(N - k) * (W / 2)];
+    const cpair h = cpair{p_pack(a.x, a.z), p_pack(a.y, a.w)}, m = cpair{p_pack(b.x, b.z), p_pack(-b.y, -b.w)};
+    const cpair e = cadd(h, m), d = cmulj(csub(h, m), w_dup(__ldg(twW + k)));
+    v[i] = cpair{p_sub(e.re, d.im), p_add(e.im, d.re)};  // e + i d
+  }
+  line_fft_pair<N, T, C, true>(v, smp, lane, t, tw);
+  const f32x2 scale = p_dup(1.f / ((float)W * (float)W));
 #pragma unroll
-  for (int i = 0; i < EW; i++) J.out[(size_t)(t + i * TW) * W + X] = v[i].x * scale;
+  for (int i = 0; i < E; i++) {
+    const size_t y = 2 * (size_t)(t + i * T);
+    *reinterpret_cast<float2*>(J.out + y * W + X) = p_unpack(p_mul(v[i].re, scale));
+    *reinterpret_cast<float2*>(J.out + (y + 1) * W + X) = p_unpack(p_mul(v[i].im, scale));
+  }
 }
 
 // ---- plan tables ----------------------------------------------------------------------------
-__global__ void k_live_otf(float* __restrict__ v, int N, const OtfTable* __restrict__ t, int att) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-  if (x >= N) return;
+// conj(OTF) over the window columns, column by column [xl][y]
+__global__ void k_live_otf(float* __restrict__ v, int N, int Xs, const OtfTable* __restrict__ t, int att) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x, xl = blockIdx.y, x = (Xs + xl) % N;
+  if (y >= N) return;
   float2 o = make_float2(0.f, 0.f);
   if (!otf_at_fast(*t, 0, freq_x(x, N), freq_y(y, N), FShift{0.f, 0.f, 0.f, 0.f}, 0, 0, att != 0, &o)) o.x = 0.f;
-  v[(size_t)y * N + x] = o.x;
+  v[(size_t)xl * N + y] = o.x;
 }
 // getDenominator x writeApoVector (the apodization from its octant table, W/2 + 1 per row)
 __global__ void k_live_wa(float* __restrict__ wa, int W, const OtfTable* __restrict__ t, ShiftSet shifts, FShiftSet fsh,
@@ -282,25 +437,39 @@ int Plan::build_live(cudaStream_t st) {
   const int N = prm.w, W = 2 * N, nA = prm.nr_dirs, nP = prm.nr_phases, nC = 2 * prm.nr_bands - 1;
   OtfTable ht;
   build_otf_table(&prm, &ht);
-  nwin = 0;
+  // window of spectrum columns inside the OTF support (all columns when it is wider), from Xs
+  plan_window(&prm, ht.cutoff / ht.vec_cpm, &nwin);
+  if (nwin > N) nwin = N;
+  const int Xs = nwin == N ? 0 : N - nwin / 2;
   std::vector<float2> coef((size_t)nA * nC * nP);
   for (int a = 0; a < nA; a++) {
     auto m = separation_coeffs(&prm, a, false);
     for (int c = 0; c < nC; c++)
       for (int q = 0; q < nP; q++) coef[(a * nC + c) * nP + q] = make_float2(m[c * nP + q].real(), m[c * nP + q].imag());
   }
-  std::vector<float2> ramps((size_t)nA * nC * 2 * N);
-  std::vector<int> off((size_t)nA * nC * 2, 0);
+  // per pos component: fractional shift ramps {x[N], y[N]} (1/N folded in), and the paste
+  // offsets and edge flags of its slot {floor(kx), floor(-ky), dx, dy}; slot 0 holds Xs
+  const int nPair = prm.nr_bands - 1;
+  std::vector<float2> ramps((size_t)nA * nPair * 2 * N);
+  std::vector<int> off((size_t)(1 + nA * nPair) * 4, 0);
+  off[0] = Xs;
   for (int a = 0; a < nA; a++)
-    for (int c = 1; c < nC; c++) {
-      const int b = (c + 1) / 2;
-      const double sg = (c % 2 == 0) ? 1.0 : -1.0;  // pos = 2b, neg = 2b-1
-      const double kx = sg * band_px(&prm, a, b), ky = sg * band_py(&prm, a, b);
+    for (int b = 1; b <= nPair; b++) {
+      const int ab = a * nPair + (b - 1);
+      const double kx = band_px(&prm, a, b), ky = band_py(&prm, a, b);
       // SimUtils.pasteAndFourierShift, fast mode (S/SimUtils.java:77-86)
       const double xFrac = kx - std::floor(kx), yFrac = -ky - std::floor(-ky);
-      off[2 * (a * nC + c)] = (int)std::floor(kx);
-      off[2 * (a * nC + c) + 1] = (int)std::floor(-ky);
-      float2* rx = &ramps[(size_t)(a * nC + c) * 2 * N];
+      int* o = &off[4 * (1 + ab)];
+      // pasteFreq takes its offsets modulo the output size: into [-N, N)
+      auto mod = [&](double f) {
+        const int m = (int)std::fmod(f, (double)W);
+        return m >= N ? m - W : (m < -N ? m + W : m);
+      };
+      o[0] = mod(std::floor(kx));
+      o[1] = mod(std::floor(-ky));
+      o[2] = xFrac != 0;
+      o[3] = yFrac != 0;
+      float2* rx = &ramps[(size_t)ab * 2 * N];
       float2* ry = rx + N;
       for (int n = 0; n < N; n++) {
         double fx = xFrac * n / N, fy = yFrac * n / N;
@@ -343,7 +512,7 @@ int Plan::build_live(cudaStream_t st) {
     FSIM_CUDA(cudaMemcpyAsync(d_damp, dv.data(), dv.size() * sizeof(float), cudaMemcpyHostToDevice, st));
   }
   FSIM_CUDA(cudaStreamSynchronize(st));
-  k_live_otf<<<dim3(div_up(N, 128), N), 128, 0, st>>>(d_masks, N, d_otf, prm.use_attenuation);
+  k_live_otf<<<dim3(div_up(N, 128), nwin), 128, 0, st>>>(d_masks, N, Xs, d_otf, prm.use_attenuation);
   // setupFilters: getDenominator(wienParam) and writeApoVector(apo, 1, 2)
   {
     float* d_apo = (float*)(b + o_apo);
@@ -359,15 +528,18 @@ int Plan::build_live(cudaStream_t st) {
   return FSIM_OK;
 }
 
+// I: column windows of band 0 and of every pos component; O: rows 0..N of the half spectrum
+static size_t live_i_bytes(const fsim_sim_param& p, int nwin) {
+  const size_t b = (size_t)(1 + p.nr_dirs * (p.nr_bands - 1)) * nwin * p.w * sizeof(float2);
+  return (b + 255) & ~(size_t)255;
+}
 size_t Plan::workspace_bytes_live() const {
-  const int N = prm.w, W = 2 * N, nC = 2 * prm.nr_bands - 1;
-  size_t I = (size_t)prm.nr_dirs * nC * N * N * sizeof(float2);
-  size_t O = (size_t)W * W * sizeof(float2);
-  return ((I + 255) & ~(size_t)255) + ((O + 255) & ~(size_t)255);
+  const size_t O = (size_t)(prm.w + 1) * 2 * prm.w * sizeof(float2);
+  return live_i_bytes(prm, nwin) + ((O + 255) & ~(size_t)255);
 }
 
 void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, char* ws) const {
-  const int N = prm.w, nC = 2 * prm.nr_bands - 1;
+  const int nC = 2 * prm.nr_bands - 1;
   j.raw = raw;
   j.out = out;
   j.widefield = wf;
@@ -376,7 +548,7 @@ void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, cha
   j.nP = prm.nr_phases;
   j.nC = nC;
   j.status = ctx().status;
-  j.nWin = 0;
+  j.nWin = nwin;
   j.bgr = 0.f;
   j.damp = d_damp;
   j.coef = d_coef;
@@ -395,31 +567,35 @@ void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, cha
   j.fwf = nullptr;
   j.wff = nullptr;
   j.Wf = nullptr;
-  size_t I = (size_t)prm.nr_dirs * nC * N * N * sizeof(float2);
   j.I = (float2*)ws;
-  j.O = (float2*)(ws + ((I + 255) & ~(size_t)255));
+  j.O = (float2*)(ws + live_i_bytes(prm, nwin));
 }
 
 template <int N>
-static int launch_live(const JobDesc* d_jobs, int njobs, int maxA, cudaStream_t st) {
+static int launch_live(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
   using P = LCfg<N>;
-  constexpr int W = P::W;
-  (void)maxA;
-  const size_t smem_d = sizeof(float2) * smem_line_elems(W, P::CD);
+  constexpr size_t E16 = sizeof(ulonglong2);
+  const size_t sm_a = E16 * P::G * P::XS, sm_b = E16 * pair_elems(N, P::CP), sm_c = LCPass<N>::SMEM,
+               sm_d = E16 * pair_elems(N, P::CD);
   static bool attr = false;
   if (!attr) {
-    FSIM_CUDA(cudaFuncSetAttribute(k_live_d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_d));
+    FSIM_CUDA(cudaFuncSetAttribute(k_live_a<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_a));
+    FSIM_CUDA(cudaFuncSetAttribute(k_live_b<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_b));
+    FSIM_CUDA(cudaFuncSetAttribute(k_live_c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_c));
+    FSIM_CUDA(cudaFuncSetAttribute(k_live_d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_d));
     attr = true;
   }
   cudaEvent_t* ev = profile_events();
   if (ev) cudaEventRecord(ev[0], st);
-  k_live_a<N><<<dim3(N / P::GA, njobs), P::GA * P::TN, 0, st>>>(d_jobs);
+  k_live_a<N><<<dim3(N / (2 * P::G), maxA + 1, njobs), P::G * P::T, sm_a, st>>>(d_jobs);
   if (ev) cudaEventRecord(ev[1], st);
-  k_live_b<N><<<dim3(N / P::CBL, njobs), P::CBL * P::TN, 0, st>>>(d_jobs);
+  k_live_b<N><<<dim3((maxWin + 2 * P::CP - 1) / (2 * P::CP), 1 + maxA * maxPair, njobs), P::CP * P::T, sm_b, st>>>(
+      d_jobs);
   if (ev) cudaEventRecord(ev[2], st);
-  k_live_c<N><<<dim3(W, njobs), P::TW, 0, st>>>(d_jobs);
+  // rows 0..N in pairs, whole groups
+  k_live_c<N><<<dim3((N / 2 + 1 + P::G - 1) / P::G, njobs), LCPass<N>::NT, sm_c, st>>>(d_jobs);
   if (ev) cudaEventRecord(ev[3], st);
-  k_live_d<N><<<dim3(W / P::CD, njobs), P::CD * P::TW, smem_d, st>>>(d_jobs);
+  k_live_d<N><<<dim3(N / P::CD, njobs), P::CD * P::T, sm_d, st>>>(d_jobs);
   if (ev) {
     cudaEventRecord(ev[4], st);
     profile_mark(4);
@@ -441,11 +617,11 @@ bool live_size_supported(int n) {
   }
 }
 
-int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, cudaStream_t st) {
+int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
   switch (n) {
 #define CASE(v) \
   case v:       \
-    return launch_live<v>(d_jobs, njobs, maxA, st);
+    return launch_live<v>(d_jobs, njobs, maxA, maxPair, maxWin, st);
     FSIM_LIVE_SIZES(CASE)
 #undef CASE
   }

@@ -154,7 +154,7 @@ int recon_batch(const fsim_job* jobs, int n, void* ws, size_t ws_bytes, cudaStre
       masks |= otf_measured(&pi->prm) ? 2 : 1;
     }
     rc = (p0->path == FSIM_PATH_LIVE)
-             ? launch_live_size(p0->prm.w, d_table + k, e - k, maxA, s)
+             ? launch_live_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, s)
              : launch_offline_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, scale_clip, masks, s);
     if (rc == FSIM_OK && p0->path == FSIM_PATH_OFFLINE) {
       bool wf = false;

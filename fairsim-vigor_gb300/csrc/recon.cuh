@@ -17,21 +17,22 @@ struct JobDesc {
   float bgr;
   const float* damp;    // N*N border fade, nullable
   const float2* coef;   // [a][c][p] separation coefficients
-  const float2* ramps;  // [a][c] {x ramp[W], y ramp[W]}  (offline) / {x ramp[N], y ramp[N]} (live)
-  const int* win;       // [a][c] {Xs, Ys} window origins (offline) / {xInt, yInt} paste offsets (live)
+  const float2* ramps;  // [a][c] {x ramp[W], y ramp[W]}  (offline) / [a][b-1] {x ramp[N], y ramp[N]} (live)
+  const int* win;       // [a][c] {Xs, Ys} window origins (offline) / {Xs, -, -, -}, then per pos component
+                        // {floor(kx), floor(-ky), dx, dy} (live.cu)
   const float* masks;   // OTF masks [band 0 (halved), neg of (a, b)][nWin column][nWin row] (offline; float2 when
-                        // cmask) / N*N conj-OTF vector (live)
+                        // cmask) / conj-OTF columns [nWin][N] (live)
   const float* wa;      // Wiener x apodization, quad layout [X/4][Y][X%4]
   const float2* nyq;    // offline: [a][b-1][x over the neg window's columns, y over its rows][nWin]: response of
                         // the neg component's odd-sample shift to the Nyquist bin (pass A)
   float2* I;            // workspace: row-transformed windows [band 0, neg of (a, b)][nWin/4][N][4] (offline);
-                        // live: [a][c] N*N row transforms
+                        // live: [band 0, pos of (a, b)][nWin/4][N][4] row, then column transforms
   float2* D;            // workspace: [a][b-1][N] Nyquist bin of every row's neg component (pass A)
   float2* G;            // workspace: [a][b-1][nWin] column transform of D (pass G, complex masks only)
   float2* Tw;           // workspace: masked column-transformed windows [band 0, neg of (a, b)][nWin column]
                         // [nWin row] (pass B1)
   float2* O;            // workspace: offline: W x N, columns 0..N-1 of the Hermitian half after pass B2
-                        // (row-major, stride N); live: W*W after the column pass
+                        // (row-major, stride N); live: rows 0..N of W, after pass LC
   float2* On;           // workspace (offline): column N of the Hermitian half, W entries
   float* clip_max;      // workspace (offline): the image maximum for CLIPSCALE.BOTH
   // widefield side outputs of the offline path (widefield.cu), run after the passes above
@@ -93,7 +94,7 @@ bool live_size_supported(int n);
 // masks: bit 0 some job of the class has real OTF masks, bit 1 some has complex ones
 int launch_offline_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip,
                         int masks, cudaStream_t st);
-int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, cudaStream_t st);
+int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st);
 // widefield and filtered widefield of the offline jobs that ask for them (widefield.cu);
 // launched after launch_offline_size on the same stream (it reuses the job workspaces)
 int launch_widefield_size(int n, const JobDesc* d_jobs, int njobs, cudaStream_t st);

@@ -38,3 +38,32 @@ def test_offline_complex_masks_vs_fp64(fs, oracle, n, pixel, apo):
     plan = fs.plan.ReconPlan(sp, path=fs.native.PATH_OFFLINE, input_type=fs.native.INPUT_F32, fade_px=10)
     got = plan.reconstruct_host(raw)
     assert rel_l2(got, oracle.recon_raw(sp, raw.astype(np.float64), fade=10, dtype=np.float64)) < 1e-5
+
+
+@pytest.mark.parametrize("n,pixel", [(64, 0.08), (64, 0.1), (128, 0.165), (256, 0.1), (384, 0.08), (512, 0.09)])
+@pytest.mark.parametrize("shift", ["fraction", "whole", "mixed"])
+def test_live_edges_vs_fp64(fs, oracle, n, pixel, shift):
+    """The live path's mirrored halves: fractional, whole-pixel and mixed shifts (the edge bins
+    of the pasted ranges differ), supports inside and beyond the raw spectrum, apodization that
+    reaches the Nyquist row and column of the output."""
+    raw, sp = _make(fs, n, n + 3, pixel, k0_frac=0.45, as_u16=True)
+    for d in range(3):
+        v = sp.dir(d)
+        x, y = v.px(1), v.py(1)
+        if shift == "whole" or (shift == "mixed" and d == 0):
+            x, y = round(x), round(y)
+        elif shift == "mixed" and d == 1:
+            x = round(x)
+        v.setPxPy(x, y)
+    plan = fs.plan.ReconPlan(sp, path=fs.native.PATH_LIVE, input_type=fs.native.INPUT_U16, fade_px=10)
+    got = plan.reconstruct_host(raw)
+    exp, _ = oracle.live_recon(sp, raw, dtype=np.float64)
+    assert rel_l2(got, exp[0]) < 1e-5
+
+
+def test_live_three_bands_vs_fp64(fs, oracle):
+    raw, sp = _make(fs, 128, 5, 0.08, k0_frac=0.45, as_u16=True, n_bands=3, n_phases=5)
+    plan = fs.plan.ReconPlan(sp, path=fs.native.PATH_LIVE, input_type=fs.native.INPUT_U16, fade_px=10)
+    got = plan.reconstruct_host(raw)
+    exp, _ = oracle.live_recon(sp, raw, dtype=np.float64)
+    assert rel_l2(got, exp[0]) < 1e-5
