@@ -79,13 +79,10 @@ struct DevBufs {
     if (rc_) return rc_;  \
   } while (0)
 
-int estimate_core(fsim_sim_param* p, const float2* const* spec, int fit_band, double fit_exclude, bool live,
-                  double* peaks_out, cudaStream_t st) {
-  TRY(validate_param(p));
-  if (!live && fit_band != 1 && fit_band != 2) {
-    set_error("Fitband neither 1 nor 2");
-    return FSIM_EINVAL;
-  }
+// Steps of the fit one vector operation at a time, direction by direction: measured OTFs and sizes
+// without a line-pair fit.
+static int fit_steps(const fsim_sim_param* p, const float2* const* spec, int fit_band, double fit_exclude, bool live,
+                     double* res, cudaStream_t st) {
   const int N = p->w, nP = p->nr_phases, nB = p->nr_bands, nC = 2 * nB - 1;
   const size_t n = (size_t)N * N;
   DevBufs bufs(st);
@@ -104,8 +101,7 @@ int estimate_core(fsim_sim_param* p, const float2* const* spec, int fit_band, do
   const double vec_cpm = ht.vec_cpm;
   // otfAtt = writeAttenuationVector(.99, 0.15*cutoff, 0, 0) (SimAlgorithm.java:65-66)
   TRY(att_device(att, N, N, vec_cpm, .99, 0.15 * ht.cutoff, 0, 0, st));
-  int rc = FSIM_OK;
-  for (int a = 0; a < p->nr_dirs && rc == FSIM_OK; a++) {
+  for (int a = 0; a < p->nr_dirs; a++) {
     auto coef = separation_coeffs(p, a, true);  // phaOff 0, fac null
     SepArgs sa{};
     sa.n_in = nP;
@@ -146,9 +142,17 @@ int estimate_core(fsim_sim_param* p, const float2* const* spec, int fit_band, do
     }
   }
   // one read of every direction's results
-  double res[8 * FSIM_MAX_DIRS];
   FSIM_CUDA(cudaMemcpyAsync(res, s.results, sizeof(double) * 8 * p->nr_dirs, cudaMemcpyDeviceToHost, st));
   FSIM_CUDA(cudaStreamSynchronize(st));
+  s.free(st);
+  otf.release(st);
+  FSIM_CUDA(cudaStreamSynchronize(st));
+  return FSIM_OK;
+}
+
+// The fitted shifts, phases and modulations of every direction from the fit's results.
+static void store_fit(fsim_sim_param* p, const double* res, int fit_band, bool live, double* peaks_out) {
+  const int nB = p->nr_bands;
   for (int a = 0; a < p->nr_dirs; a++) {
     const double* r = res + 8 * a;
     double fit[4] = {r[0], r[1], r[2], r[3]};
@@ -178,10 +182,30 @@ int estimate_core(fsim_sim_param* p, const float2* const* spec, int fit_band, do
     if (peaks_out)
       for (int i = 0; i < 4; i++) peaks_out[4 * a + i] = fit[i];
   }
-  s.free(st);
-  otf.release(st);
-  FSIM_CUDA(cudaStreamSynchronize(st));
-  return rc;
+}
+
+static int check_fit(const fsim_sim_param* p, int fit_band, bool live) {
+  TRY(validate_param(p));
+  if (!live && fit_band != 1 && fit_band != 2) {
+    set_error("Fitband neither 1 nor 2");
+    return FSIM_EINVAL;
+  }
+  return FSIM_OK;
+}
+
+int estimate_core(fsim_sim_param* p, const float2* const* spec, int fit_band, double fit_exclude, bool live,
+                  double* peaks_out, cudaStream_t st) {
+  TRY(check_fit(p, fit_band, live));
+  double res[8 * FSIM_MAX_DIRS];
+  if (fit_pairs_supported(p, 0)) {
+    FitSource src;
+    src.spec = spec;
+    TRY(fit_pairs(p, src, fit_band, fit_exclude, live, res, st));
+  } else {
+    TRY(fit_steps(p, spec, fit_band, fit_exclude, live, res, st));
+  }
+  store_fit(p, res, fit_band, live, peaks_out);
+  return FSIM_OK;
 }
 
 // raw frames on the device -> spectra (damp, forward FFT), as the GUI / live code prepares them
@@ -198,6 +222,30 @@ static int raw_to_spectra(const fsim_sim_param* p, const void* raw, int input_u1
   }
   TRY(raw_to_cplx_device(spec, raw, input_u16, damp, n, frames, st));
   return fft2d_device(spec, N, N, false, st, frames);
+}
+
+static int estimate_raw(fsim_sim_param* p, const void* raw, int input_u16, int fade_px, int fit_band,
+                        double fit_exclude, bool live, double* peaks_out, cudaStream_t st) {
+  TRY(check_fit(p, fit_band, live));
+  if (fit_pairs_supported(p, fade_px)) {
+    FitSource src;
+    src.raw = raw;
+    src.u16 = input_u16;
+    src.fade_px = fade_px;
+    double res[8 * FSIM_MAX_DIRS];
+    TRY(fit_pairs(p, src, fit_band, fit_exclude, live, res, st));
+    store_fit(p, res, fit_band, live, peaks_out);
+    return FSIM_OK;
+  }
+  const int frames = p->nr_dirs * p->nr_phases;
+  const size_t n = (size_t)p->w * p->w;
+  DevBufs bufs(st);
+  float2* spec;
+  TRY(bufs.get(&spec, sizeof(float2) * n * frames));
+  TRY(raw_to_spectra(p, raw, input_u16, fade_px, spec, bufs, st));
+  std::vector<const float2*> ptrs(frames);
+  for (int i = 0; i < frames; i++) ptrs[i] = spec + i * n;
+  return estimate_core(p, ptrs.data(), fit_band, fit_exclude, live, peaks_out, st);
 }
 
 // ---- the op-by-op reconstruction -------------------------------------------------------------
@@ -599,32 +647,15 @@ int fsim_estimate_raw(fsim_sim_param* p, const void* raw_device, int input_type,
   NEED_INIT();
   TRY(validate_param(p));
   FSIM_REQUIRE(raw_device, FSIM_EINVAL, "null raw pointer");
-  cudaStream_t st = ctx().stream;
-  const int frames = p->nr_dirs * p->nr_phases;
-  const size_t n = (size_t)p->w * p->w;
-  DevBufs bufs(st);
-  float2* spec;
-  TRY(bufs.get(&spec, sizeof(float2) * n * frames));
-  TRY(raw_to_spectra(p, raw_device, input_type == FSIM_INPUT_U16, fade_px, spec, bufs, st));
-  std::vector<const float2*> ptrs(frames);
-  for (int i = 0; i < frames; i++) ptrs[i] = spec + i * n;
-  return estimate_core(p, ptrs.data(), fit_band, fit_exclude, false, peaks_out, st);
+  return estimate_raw(p, raw_device, input_type == FSIM_INPUT_U16, fade_px, fit_band, fit_exclude, false, peaks_out,
+                      ctx().stream);
 }
 
 int fsim_live_refit(fsim_sim_param* p, const uint16_t* raw_device, double* peaks_out) {
   NEED_INIT();
   TRY(validate_param(p));
   FSIM_REQUIRE(raw_device, FSIM_EINVAL, "null raw pointer");
-  cudaStream_t st = ctx().stream;
-  const int frames = p->nr_dirs * p->nr_phases;
-  const size_t n = (size_t)p->w * p->w;
-  DevBufs bufs(st);
-  float2* spec;
-  TRY(bufs.get(&spec, sizeof(float2) * n * frames));
-  TRY(raw_to_spectra(p, raw_device, 1, 10, spec, bufs, st));
-  std::vector<const float2*> ptrs(frames);
-  for (int i = 0; i < frames; i++) ptrs[i] = spec + i * n;
-  return estimate_core(p, ptrs.data(), 1, .8, true, peaks_out, st);
+  return estimate_raw(p, raw_device, 1, 10, 1, .8, true, peaks_out, ctx().stream);
 }
 
 int fsim_rl_deconvolve(fsim_vec* img, const fsim_vec* otf, int steps, int input_in_freq_space) {

@@ -20,6 +20,10 @@ template <class T>
 cudaError_t dev_alloc(T** p, size_t bytes) {
   return dev_alloc(reinterpret_cast<void**>(p), bytes);
 }
+// Stream-ordered scratch (freed with cudaFreeAsync) from a pool that keeps up to 512 MiB
+// between calls: without it every call maps and unmaps its memory. The pool serves any number of
+// threads and streams (the runtime orders reuse), and its idle memory is returned when another
+// allocation of the library would fail.
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t st);
 template <class T>
 cudaError_t dev_alloc_async(T** p, size_t bytes, cudaStream_t st) {

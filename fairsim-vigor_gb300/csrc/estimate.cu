@@ -36,34 +36,6 @@ __device__ __forceinline__ float2 cdiv_java(float2 a, float2 b) {
 // in the integer r^2, so it is decided by the thresholds r2_lo / r2_hi that the host finds with
 // the reference's double expression (mx == 0 keeps the expression itself). Weight limits
 // compare floats with wlf, the smallest float >= wl ((double)f < wl exactly when f < wlf).
-struct CrParams {  // commonRegion's shift and its ratio-cut thresholds
-  double kx, ky;
-  FShift kf;
-  long long r2_lo, r2_hi;
-  int mx_zero;
-};
-// The thresholds of the ratio cut for |k| = mx: ratio = sqrt((double)r^2) / mx is
-// non-decreasing in the integer r^2, so "ratio < dist" holds below r2_lo and
-// "ratio > 1 - dist" above r2_hi (bisection; sqrt and division are correctly rounded on the
-// host and the device alike, so both find the same integers).
-// The search starts at the estimate (dist * mx)^2 and steps until the predicate flips, a few
-// evaluations (the device runs it on one thread, where a bisection's chain of FP64 square
-// roots and divisions took tens of microseconds).
-__host__ __device__ inline void cr_thresholds(double mx, double dist, long long r2max, long long* r2_lo,
-                                              long long* r2_hi) {
-  auto below = [&](long long m) { return sqrt((double)m) / mx < dist; };       // the inner cut
-  auto above = [&](long long m) { return sqrt((double)m) / mx > (1 - dist); };  // the outer cut
-  auto clampr = [&](double v) { return v < 0 ? 0LL : (v > (double)r2max ? r2max : (long long)v); };
-  long long e = clampr(dist * mx * (dist * mx));  // first r2 with !below
-  while (e <= r2max && below(e)) e++;
-  while (e > 0 && !below(e - 1)) e--;
-  *r2_lo = e;
-  e = clampr((1 - dist) * mx * ((1 - dist) * mx));  // last r2 with !above
-  while (e >= 0 && above(e)) e--;
-  while (e < r2max && !above(e + 1)) e++;
-  *r2_hi = e;
-}
-
 __device__ __forceinline__ void common_region_px(float2* __restrict__ b0, float2* __restrict__ b1, int w, int h,
                                                  const OtfTable* __restrict__ t, const CrParams& cp, double dist,
                                                  float wlf, int divide, int bn0, int bn1, int x, int y) {

@@ -269,12 +269,18 @@ int apo_device(float* out, int cplx, int W, int H, double vec_cpm, double cutoff
 // Unshifted on a square grid the attenuation depends on (|x~|, |y~|) only, symmetrically:
 // evaluated in double once per octant point 0 <= j <= i <= n/2 (the same expression as
 // k_att_vector, so the same bits) and spread over the grid.
-__global__ void k_att_octant(float* __restrict__ q, int h2, double vec_cpm, double str, double fwhm) {
+__global__ void k_att_octant(float* __restrict__ q, int h2, double vec_cpm, double str, double fwhm, float unit) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
   if (j > i) return;
+  // beyond 6.8 widths 1 - str * exp(-u), u > 23, rounds to 1.0f (|str| <= 1): FP64 only inside
+  // (unit: the exponent one pixel from the centre)
+  if ((float)(i * i + j * j) * unit > 23.f && fabs(str) <= 1) {
+    q[(size_t)i * (h2 + 1) + j] = 1.f;
+    return;
+  }
+  const double s = fwhm / 2.355;
   const double rad = d_hypot_java((double)i, (double)j);
   const double dist = __dmul_rn(rad, vec_cpm);
-  const double s = fwhm / 2.355;
   const double g = exp(-__dmul_rn(dist, dist) / __dmul_rn(2.0, __dmul_rn(s, s)));
   q[(size_t)i * (h2 + 1) + j] = (float)__dsub_rn(1.0, __dmul_rn(str, g));
 }
@@ -291,7 +297,8 @@ int att_device(float* out, int w, int h, double vec_cpm, double str, double fwhm
     const int h2 = w / 2;
     float* q = nullptr;
     FSIM_CUDA(fsim::dev_alloc_async(&q, sizeof(float) * (size_t)(h2 + 1) * (h2 + 1), st));
-    k_att_octant<<<dim3(div_up(h2 + 1, 128), h2 + 1), 128, 0, st>>>(q, h2, vec_cpm, str, fwhm);
+    k_att_octant<<<dim3(div_up(h2 + 1, 128), h2 + 1), 128, 0, st>>>(
+        q, h2, vec_cpm, str, fwhm, (float)(vec_cpm * vec_cpm / (2 * (fwhm / 2.355) * (fwhm / 2.355))));
     k_att_expand<<<g, 128, 0, st>>>(out, w, q);
     FSIM_CHECK_LAUNCH();
     FSIM_CUDA(cudaFreeAsync(q, st));

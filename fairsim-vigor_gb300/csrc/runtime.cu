@@ -30,32 +30,51 @@ static std::atomic<int> g_fail_alloc{0};
 // The setting of fsim_debug_b2_staging, which no longer selects anything
 static std::atomic<int> g_b2_staging{1};
 
-cudaError_t dev_alloc(void** p, size_t bytes) {
+// true when the armed allocation failure falls on this allocation
+static bool fail_injected() {
   int n = g_fail_alloc.load();
-  while (n > 0) {
-    if (g_fail_alloc.compare_exchange_weak(n, n - 1)) {
-      if (n == 1) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-      }
-      break;
-    }
-  }
-  return cudaMalloc(p, bytes);
+  while (n > 0)
+    if (g_fail_alloc.compare_exchange_weak(n, n - 1)) return n == 1;
+  return false;
+}
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool = nullptr;
+constexpr unsigned long long kPoolKeep = 512ull << 20;  // bytes the pool may keep idle
+// returns the pool's idle memory; false when there is no pool
+static bool trim_pool() {
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  if (!g_pool) return false;
+  (void)cudaGetLastError();  // the failed allocation's
+  return cudaDeviceSynchronize() == cudaSuccess && cudaMemPoolTrimTo(g_pool, 0) == cudaSuccess;
+}
+
+cudaError_t dev_alloc(void** p, size_t bytes) {
+  *p = nullptr;
+  if (fail_injected()) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && trim_pool()) e = cudaMalloc(p, bytes);
+  return e;
 }
 
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t st) {
-  int n = g_fail_alloc.load();
-  while (n > 0) {
-    if (g_fail_alloc.compare_exchange_weak(n, n - 1)) {
-      if (n == 1) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-      }
-      break;
+  *p = nullptr;
+  if (fail_injected()) return cudaErrorMemoryAllocation;
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if (!g_pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = ctx().device;
+      cudaError_t e = cudaMemPoolCreate(&g_pool, &props);
+      unsigned long long keep = kPoolKeep;
+      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(g_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) return e;
     }
+    pool = g_pool;
   }
-  return cudaMallocAsync(p, bytes, st);
+  return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
 static std::mutex g_mu;
