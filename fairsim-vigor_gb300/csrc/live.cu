@@ -28,8 +28,8 @@
 // The OTF also zeroes every column beyond its support: only a window of columns leaves LA.
 // Rows (LA, LC) and columns (LB, LD) are transformed two at a time (fft_pair.cuh). Bound by the
 // shared-memory pipe and instruction issue of 11.6k transforms of length N per 512^2 3x3 stack (26k
-// with every component and the full grid): 64 stacks in 1116 us on GB300, 2382 us before; one
-// stack 66.7 us, 109 before.
+// with every component and the full grid): 64 stacks in 1087 us on GB300, 2382 us before; one
+// stack 62.6 us, 109 before.
 #include <cmath>
 #include <vector>
 
@@ -54,9 +54,13 @@ struct LCfg {
   static constexpr int G = T >= 64 ? 1 : 64 / T;    // row pairs per block, passes LA and LC
   static constexpr int CP = 2;                      // column pairs per block, pass LB
   static constexpr int CD = N >= 2048 ? 2 : 4;      // column pairs per block, pass LD
-  static constexpr int R = E <= 8 ? 80 : 128;       // registers per thread
-  static constexpr int blocks(int threads) {
-    const int n = threads < 32 ? 32 : threads, b = 65536 / (n * R);
+  // Registers per thread at 8 elements: 80, but 96 in pass LA, which keeps two frames' pixels in
+  // flight while it mixes (64 x 512^2: 361 -> 318 us; three frames 342), and 128 in pass LC, which
+  // loads the next contribution during a transform (474 -> 436 us; 531 at 80, where it spills).
+  static constexpr int R = E <= 8 ? 80 : 128;
+  static constexpr int RA = 96, RC = 128, F = 2;
+  static constexpr int blocks(int threads, int regs8 = 80) {
+    const int n = threads < 32 ? 32 : threads, b = 65536 / (n * (E <= 8 ? regs8 : R));
     return b < 1 ? 1 : (b > 32 ? 32 : b);
   }
   static constexpr int XS = pair_elems(N, 1);       // exchange buffer of one pair
@@ -72,7 +76,7 @@ __device__ __forceinline__ int live_col(int m, int Xs) {
 // blockIdx.y < nA: the pos components of that angle; blockIdx.y == nA: band 0 of all angles, and
 // the widefield.
 template <int N>
-__global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N>::G* LCfg<N>::T))
+__global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N>::G* LCfg<N>::T, LCfg<N>::RA))
     k_live_a(const JobDesc* __restrict__ jobs) {
   using P = LCfg<N>;
   constexpr int T = P::T, G = P::G, E = P::E;
@@ -104,6 +108,25 @@ __global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N
       for (int i = 0; i < E; i++) v[i] = p_mul(v[i], p_pack(__ldg(d + i * T), __ldg(d + N + i * T)));
     }
   };
+  // frames f0 .. f0 + nf - 1, several frames' loads in flight at once
+  auto mix = [&](int f0, int nf, auto add) {
+    constexpr int F = P::F;
+    int f = f0;
+#pragma unroll 1
+    for (; f + F <= f0 + nf; f += F) {
+      f32x2 v[F][E];
+#pragma unroll
+      for (int k = 0; k < F; k++) px_rows(f + k, v[k]);
+#pragma unroll
+      for (int k = 0; k < F; k++) add(v[k], f + k);
+    }
+#pragma unroll 1
+    for (; f < f0 + nf; f++) {
+      f32x2 v[E];
+      px_rows(f, v);
+      add(v, f);
+    }
+  };
   // both rows' value of the window columns, to the quad layout [xl/4][y][xl%4]
   cpair x[E];  // element t + i*T of both rows, in registers through the transform
   auto put = [&](int slot) {
@@ -127,17 +150,15 @@ __global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N
       x[i] = cp_zero();
       wf[i] = 0ull;
     }
-#pragma unroll 1
-    for (int f = 0; f < nA * nP; f++) {
-      f32x2 v[E];
-      px_rows(f, v);
+    auto add = [&](const f32x2 (&v)[E], int f) {
       const wpair m = w_dup(__ldg(J.coef + (f / nP) * nC * nP + f % nP));
 #pragma unroll
       for (int i = 0; i < E; i++) {
         wf[i] = p_add(wf[i], v[i]);
         x[i] = cpair{p_fma(m.x, v[i], x[i].re), p_fma(m.y, v[i], x[i].im)};
       }
-    }
+    };
+    mix(0, nA * nP, add);
     if (J.widefield) {
       const f32x2 sc = p_dup(1.f / (float)(nA * nP));
 #pragma unroll
@@ -155,14 +176,11 @@ __global__ void __launch_bounds__(LCfg<N>::G* LCfg<N>::T, LCfg<N>::blocks(LCfg<N
     const float2* coef = J.coef + (a * nC + 2 * b) * nP;
 #pragma unroll
     for (int i = 0; i < E; i++) x[i] = cp_zero();
-#pragma unroll 1
-    for (int p = 0; p < nP; p++) {
-      f32x2 v[E];
-      px_rows(a * nP + p, v);
-      const wpair m = w_dup(__ldg(coef + p));
+    mix(a * nP, nP, [&](const f32x2 (&v)[E], int f) {
+      const wpair m = w_dup(__ldg(coef + (f - a * nP)));
 #pragma unroll
       for (int i = 0; i < E; i++) x[i] = cpair{p_fma(m.x, v[i], x[i].re), p_fma(m.y, v[i], x[i].im)};
-    }
+    });
     line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
     put(1 + a * nPair + (b - 1));
   }
@@ -226,7 +244,7 @@ struct LCPass {
   static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)P::G * GS;
 };
 template <int N>
-__global__ void __launch_bounds__(LCPass<N>::NT, LCfg<N>::blocks(LCPass<N>::NT))
+__global__ void __launch_bounds__(LCPass<N>::NT, LCfg<N>::blocks(LCPass<N>::NT, LCfg<N>::RC))
     k_live_c(const JobDesc* __restrict__ jobs) {
   using P = LCfg<N>;
   constexpr int W = P::W, T = P::T, E = P::E, G = P::G;
@@ -243,89 +261,111 @@ __global__ void __launch_bounds__(LCPass<N>::NT, LCfg<N>::blocks(LCPass<N>::NT))
   auto wrap = [](int v) { return v < 0 ? v + W : (v >= W ? v - W : v); };
 #pragma unroll
   for (int i = 0; i < 2 * E; i++) acc[t + i * T] = make_ulonglong2(0ull, 0ull);
-  // One contribution: rows q0 and q0 + d of the slot (relative to its origin; d = -1 mirrored).
-  // u[h] are the weights of the direct and the mirrored range for row h.
-  cpair x[E];
-  auto load_row = [&](const float2* I, int q, bool on, float2 (&v)[E]) {
-    const int ys = q < 0 ? q + N : (q >= N ? q - N : q);
+  // Contribution k: slot k / 2, direct (even k) or mirrored (odd), from the slot's rows q[0], q[1]
+  // relative to its origin. Rows are in the pos range [-N/2, N/2 - 1], in the neg range
+  // [dy - N/2 + 1, dy + N/2] (band 0: the pos range only, its mirror image included); wp, wn: weights
+  // of an element inside the pos / the neg x range.
+  struct Part {
+    int sl, mir, xi, dx, q[2];
+    float wp[2], wn[2];
+    bool any;
+  };
+  auto part = [&](int k) {
+    Part c;
+    c.sl = k >> 1;
+    c.mir = k & 1;
+    const int* w = J.win + 4 * c.sl;  // slot 0: (Xs, 0, -, -); pairs: floor(kx), floor(-ky), dx, dy
+    const int yi = c.sl ? w[1] : 0, dy = c.sl ? w[3] : 0;
+    c.xi = c.sl ? w[0] : 0;
+    c.dx = c.sl ? w[2] : 0;
+    c.any = false;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      int q = (c.mir ? -(Y0 + h) : Y0 + h) - yi;
+      if (q < -N) q += W;  // floor(k) shifts reach beyond the grid's half
+      else if (q >= N) q -= W;
+      const bool in_p = q >= -N / 2 && q <= N / 2 - 1, in_n = c.sl && q >= dy - N / 2 + 1 && q <= dy + N / 2;
+      c.q[h] = q;
+      c.wp[h] = in_p ? (c.sl ? 0.5f : 1.f) : 0.f;
+      c.wn[h] = in_n ? 0.5f : 0.f;
+      c.any = c.any || in_p || in_n;
+    }
+    return c;
+  };
+  // the next contribution at or after k that some row pair of the block takes part in
+  auto next = [&](int k) {
+    for (; k < 2 * nS; k++) {
+      const bool any = part(k).any;
+      if (P::G == 1 ? any : (bool)__syncthreads_or(any)) break;
+    }
+    return k;
+  };
+  auto load = [&](int k, cpair (&v)[E]) {
+    const Part c = part(k);
+    const float2* I = J.I + (size_t)c.sl * nWin * N;
+    const bool on0 = c.wp[0] + c.wn[0] > 0.f, on1 = c.wp[1] + c.wn[1] > 0.f;
+    const int y0 = c.q[0] < 0 ? c.q[0] + N : c.q[0], y1 = c.q[1] < 0 ? c.q[1] + N : c.q[1];
 #pragma unroll
     for (int i = 0; i < E; i++) {
       const int xl = live_col<N>(t + i * T, Xs);
-      v[i] = (on && xl < nWin) ? __ldg(I + ((size_t)(xl >> 2) * N + ys) * 4 + (xl & 3)) : make_float2(0.f, 0.f);
+      const size_t col = (size_t)(xl >> 2) * N * 4 + (xl & 3);
+      const float2 z = make_float2(0.f, 0.f);
+      v[i] = cp_make(on0 && xl < nWin ? __ldg(I + col + (size_t)y0 * 4) : z,
+                     on1 && xl < nWin ? __ldg(I + col + (size_t)y1 * 4) : z);
     }
   };
-  for (int sl = 0; sl < nS; sl++) {
-    const float2* I = J.I + (size_t)sl * nWin * N;
-    const int* w = J.win + 4 * sl;  // slot 0: (Xs, 0, -, -); pairs: floor(kx), floor(-ky), dx, dy
-    const int xi = sl ? w[0] : 0, yi = sl ? w[1] : 0, dx = sl ? w[2] : 0, dy = sl ? w[3] : 0;
-    for (int mir = 0; mir < 2; mir++) {
-      // Rows of the slot, relative to its origin: in the pos range [-N/2, N/2 - 1], in the neg
-      // range [dy - N/2 + 1, dy + N/2] (band 0: the pos range only, its mirror image included).
-      int q[2];
-      float wp[2], wn[2];  // weights of an element inside the pos / the neg x range
-      bool any = false;
+  cpair x[E], xn[E];
+  int k = next(0);
+  if (k < 2 * nS) load(k, xn);
+  while (k < 2 * nS) {
+    const Part c = part(k);
+    const int sl = c.sl, mir = c.mir, xi = c.xi, dx = c.dx;
+#pragma unroll
+    for (int i = 0; i < E; i++) x[i] = xn[i];
+    k = next(k + 1);
+    if (k < 2 * nS) load(k, xn);  // in flight during this contribution's transforms
+    __syncthreads();              // the previous contribution's sums are complete
+    if (sl) {
+      line_fft_pair<N, T, 1, true>(x, s, 0, t, tw);
+      const float2* rx = J.ramps + (size_t)(sl - 1) * 2 * N;
+#pragma unroll
+      for (int i = 0; i < E; i++) x[i] = cmul(x[i], w_dup(__ldg(rx + t + i * T)));
+      line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
+    }
+    // v at p = px; sp, sn: inside the pos / the neg range along x
+    auto add = [&](int px, bool sp, bool sn, cpair v) {
+      int X = xi + px;
+      if (mir) X = -X;
+      X = wrap(wrap(X));
+      float u[2];
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        q[h] = (mir ? -(Y0 + h) : Y0 + h) - yi;
-        if (q[h] < -N) q[h] += W;  // floor(k) shifts reach beyond the grid's half
-        else if (q[h] >= N) q[h] -= W;
-        const bool in_p = q[h] >= -N / 2 && q[h] <= N / 2 - 1;
-        const bool in_n = q[h] >= dy - N / 2 + 1 && q[h] <= dy + N / 2;
-        wp[h] = sl ? (in_p ? 0.5f : 0.f) : (in_p ? 1.f : 0.f);
-        wn[h] = sl && in_n ? 0.5f : 0.f;
-        any = any || in_p || (sl && in_n);
-      }
-      any = __syncthreads_or(any);  // the same for every row pair of the block; orders the sums, too
-      if (!any) continue;
-      {
-        float2 r0[E], r1[E];
-        load_row(I, q[0], wp[0] + wn[0] > 0.f, r0);
-        load_row(I, q[1], wp[1] + wn[1] > 0.f, r1);
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = cp_make(r0[i], r1[i]);
-      }
-      if (sl) {
-        line_fft_pair<N, T, 1, true>(x, s, 0, t, tw);
-        const float2* rx = J.ramps + (size_t)(sl - 1) * 2 * N;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = cmul(x[i], w_dup(__ldg(rx + t + i * T)));
-        line_fft_pair<N, T, 1, false>(x, s, 0, t, tw);
-      }
-      // v at p = px; sp, sn: inside the pos / the neg range along x
-      auto add = [&](int px, bool sp, bool sn, cpair v) {
-        int X = xi + px;
-        if (mir) X = -X;
-        X = wrap(wrap(X));
-        float u[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          float fp = 1.f, fn = 1.f;
-          if (X == N || Y0 == N) {
-            // The Nyquist column and row are their own mirror images, but Wiener and apodization
-            // differ between the coordinates -N and +N: each part is weighted here, at its own
-            // position (the pos range's at floor(k) + p, the neg range's at the mirrored one).
-            const float f0 = __ldg(wa + (size_t)(Y0 + h) * W + X);
-            const float f1 = __ldg(wa + (size_t)wrap(-(Y0 + h)) * W + wrap(-X));
-            fp = mir ? f1 : f0;
-            fn = mir ? f0 : f1;
-          }
-          u[h] = (sp ? wp[h] * fp : 0.f) + (sn ? wn[h] * fn : 0.f);
+        float fp = 1.f, fn = 1.f;
+        if (X == N || Y0 == N) {
+          // The Nyquist column and row are their own mirror images, but Wiener and apodization
+          // differ between the coordinates -N and +N: each part is weighted here, at its own
+          // position (the pos range's at floor(k) + p, the neg range's at the mirrored one).
+          const float f0 = __ldg(wa + (size_t)(Y0 + h) * W + X);
+          const float f1 = __ldg(wa + (size_t)wrap(-(Y0 + h)) * W + wrap(-X));
+          fp = mir ? f1 : f0;
+          fn = mir ? f0 : f1;
         }
-        const f32x2 f = p_pack(u[0], u[1]);
-        ulonglong2 o = acc[X];
-        o.x = p_fma(v.re, f, o.x);
-        o.y = p_fma(v.im, mir ? p_neg(f) : f, o.y);
-        acc[X] = o;
-      };
-      // element m at p = m~ (signed), and, for the bins on the edge, at m~ + N in the neg range
-      // (no two elements of a contribution meet)
-#pragma unroll
-      for (int i = 0; i < E; i++) {
-        const int m = t + i * T, px = m < N / 2 ? m : m - N;
-        const bool in_n = px >= dx - N / 2 + 1;
-        add(px, true, in_n, x[i]);
-        if (sl && !in_n) add(px + N, false, true, x[i]);
+        u[h] = (sp ? c.wp[h] * fp : 0.f) + (sn ? c.wn[h] * fn : 0.f);
       }
+      const f32x2 f = p_pack(u[0], u[1]);
+      ulonglong2 o = acc[X];
+      o.x = p_fma(v.re, f, o.x);
+      o.y = p_fma(v.im, mir ? p_neg(f) : f, o.y);
+      acc[X] = o;
+    };
+    // element m at p = m~ (signed), and, for the bins on the edge, at m~ + N in the neg range
+    // (no two elements of a contribution meet)
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+      const int m = t + i * T, px = m < N / 2 ? m : m - N;
+      const bool in_n = px >= dx - N / 2 + 1;
+      add(px, true, in_n, x[i]);
+      if (sl && !in_n) add(px + N, false, true, x[i]);
     }
   }
   __syncthreads();
