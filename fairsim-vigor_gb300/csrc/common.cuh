@@ -73,6 +73,30 @@ __host__ __device__ __forceinline__ float2 cconjf(float2 a) { return make_float2
 __host__ __device__ __forceinline__ int freq_x(int x, int w) { return x < w / 2 ? x : x - w; }
 __host__ __device__ __forceinline__ int freq_y(int y, int h) { return y < h / 2 ? -y : h - y; }
 
+// ---- programmatic dependent launch --------------------------------------------------------
+// The passes of a small batch last a few microseconds each, as long as the drain and launch between
+// them. A pass launched as a dependent one starts while the last blocks of the previous pass run;
+// its blocks wait in pdl_wait() until that pass has completed and its writes are visible, before
+// they touch anything it wrote. pdl_trigger() lets the next pass start. A block that leaves early
+// waits too, so that a pass never completes before the one it follows.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_pass(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                               A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace fsim

@@ -155,7 +155,7 @@ int recon_batch(const fsim_job* jobs, int n, void* ws, size_t ws_bytes, cudaStre
     }
     rc = (p0->path == FSIM_PATH_LIVE)
              ? launch_live_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, s)
-             : launch_offline_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, scale_clip, masks, s);
+             : launch_offline_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, scale_clip, masks, nfork == 0, s);
     if (rc == FSIM_OK && p0->path == FSIM_PATH_OFFLINE) {
       bool wf = false;
       for (int i = k; i < e; i++) wf = wf || jobs[order[i]].widefield || jobs[order[i]].filtered_widefield;

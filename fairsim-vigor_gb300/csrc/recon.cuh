@@ -92,8 +92,9 @@ bool live_size_supported(int n);
 // of the batch's datasets of size n (they bound the grids; extra blocks exit at once)
 // scale_clip: some job of the class asks for CLIPSCALE.BOTH (one more pass scales its image)
 // masks: bit 0 some job of the class has real OTF masks, bit 1 some has complex ones
+// alone: no other size class of the batch runs beside this one
 int launch_offline_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip,
-                        int masks, cudaStream_t st);
+                        int masks, bool alone, cudaStream_t st);
 int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st);
 // widefield and filtered widefield of the offline jobs that ask for them (widefield.cu);
 // launched after launch_offline_size on the same stream (it reuses the job workspaces)

@@ -19,6 +19,7 @@
 #include "filters.cuh"
 #include "otf.cuh"
 #include "recon.cuh"
+#include "runtime.cuh"
 
 // Register budgets (registers per thread) of passes A, B1 and B2 at 8 elements per thread: two
 // lines of 8 complex values are 32 registers, a butterfly's operands and twiddles the rest.
@@ -129,7 +130,13 @@ struct PassA {
   static constexpr int XS = pair_elems(N, 1);
   static constexpr int GS = XS + N;  // shared-memory elements per group
   static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)G * GS;
-  static constexpr int MINB = pair_min_blocks(NT, EN, FSIM_PA_REGS);
+  // Frames whose pixels are in flight at once while a thread mixes them. Three frames take 96
+  // registers where one takes 80, but blocks of 64 threads lose little residence by it: 64 x 512^2
+  // 491 -> 473 us. Larger blocks lose more (2048^2: two blocks per SM instead of three, the whole
+  // reconstruction 464 -> 497 us; 8 x 1024^2 750 -> 756), and 12 elements per thread leave no room
+  // (8 x 768^2 594 -> 596).
+  static constexpr int F = (NT <= 64 && EN <= 8) ? 3 : 1;
+  static constexpr int MINB = pair_min_blocks(NT, EN, F > 1 ? 96 : FSIM_PA_REGS);
   static_assert(N % RB == 0, "whole blocks of rows");
 };
 
@@ -149,6 +156,7 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   ulonglong2* s = smp + g * PA::GS;
   const float2* twN = g_stw + stw_offset(N, EN);  // stage table, read through L1
   const float2* twW = g_tw + tw_offset(W);
+  pdl_trigger();
   const JobDesc* jg = jobs + blockIdx.z;
   load_job(&J, jg, tid, NT);
   // the counts and the separation coefficients straight from the descriptor in global
@@ -178,17 +186,30 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   auto mix = [&](int f0, int nf, const float2* c) {
 #pragma unroll
     for (int i = 0; i < EN; i++) x[i] = cp_zero();
-#pragma unroll 1
-    for (int p = 0; p < nf; p++) {
-      float v[2][EN];
-      raw_rows<N, EN, T>(J, (size_t)(f0 + p) * frame, row, t, v);
-      const wpair m = w_dup(c[p]);
+    auto add = [&](float (&v)[2][EN], float2 k) {
+      const wpair m = w_dup(k);
 #pragma unroll
       for (int i = 0; i < EN; i++) {
         const f32x2 r = p_pack(v[0][i], v[1][i]);
         x[i].re = p_fma(m.x, r, x[i].re);
         x[i].im = p_fma(m.y, r, x[i].im);
       }
+    };
+    constexpr int F = PA::F;
+    int p = 0;
+#pragma unroll 1
+    for (; p + F <= nf; p += F) {
+      float v[F][2][EN];
+#pragma unroll
+      for (int f = 0; f < F; f++) raw_rows<N, EN, T>(J, (size_t)(f0 + p + f) * frame, row, t, v[f]);
+#pragma unroll
+      for (int f = 0; f < F; f++) add(v[f], c[p + f]);
+    }
+#pragma unroll 1
+    for (; p < nf; p++) {
+      float v[2][EN];
+      raw_rows<N, EN, T>(J, (size_t)(f0 + p) * frame, row, t, v);
+      add(v, c[p]);
     }
     damp_rows<N, EN, T>(J, row, t, x);
   };
@@ -397,8 +418,10 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   const int lt = threadIdx.x, lane = lt % CP, t = lt / CP;
   __shared__ JobDesc J;
   extern __shared__ ulonglong2 smp[];
-  load_job(&J, jobs + blockIdx.y, lt, NT);
+  load_job(&J, jobs + blockIdx.y, lt, NT);  // written before pass A
   __syncthreads();
+  pdl_wait();
+  pdl_trigger();  // pass B1 may start: pass A is complete
   if ((J.cmask != 0) != CM) return;  // the other launch's job (uniform per block)
   const int nWin = J.nWin;
   if ((int)blockIdx.x * CB >= nWin) return;  // uniform per block
@@ -436,11 +459,17 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   const float2* twN = g_stw + stw_offset(N, EN);
   const float2* twW = g_tw + tw_offset(W);
   load_job(&J, jobs + blockIdx.z, lt, NT);
+  pdl_trigger();
   __syncthreads();
-  if ((J.cmask != 0) != CM) return;  // the other launch's job (uniform per block)
   const int nC = J.nC, nWin = J.nWin, nPair = (nC - 1) / 2;
   const int comp = 1 + blockIdx.y;  // 1 + a*nPair + (b-1): neg of (a, b)
-  if (comp > J.nA * nPair || (int)blockIdx.x * CB >= nWin) return;  // uniform per block
+  // No block of this pass is launched before every block of k_pass_b0 has returned from its wait,
+  // so pass A is complete by now, as the job table is; k_pass_b0's own work is not read here and is
+  // only waited for before the block ends (one 256^2 stack: 34 us, 45 with the wait up here).
+  if ((J.cmask != 0) != CM /* the other launch's job */ || comp > J.nA * nPair || (int)blockIdx.x * CB >= nWin) {
+    pdl_wait();
+    return;  // uniform per block
+  }
   const int xl = blockIdx.x * CB + 2 * lane;  // and xl + 1; nWin is a multiple of 4: both are inside
   const size_t col = ((size_t)comp * nWin + xl) * nWin;
   cpair x[EN];  // element t + i*T of this lane's columns, in registers through the transforms
@@ -523,6 +552,7 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
       if (yl + N < nWin) finish(yl + N, csub(e, o));
     }
   }
+  pdl_wait();
 }
 
 // ---- pass B2: Hermitian sum over components, Wiener x apodization, inverse along y -------------
@@ -555,6 +585,8 @@ __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::
   const float2* twN = g_stw + stw_offset(N, EN);
   const float2* twW = g_tw + tw_offset(W);
   load_job(&J, jobs + blockIdx.y, lt, NT);
+  pdl_trigger();
+  pdl_wait();
   __syncthreads();
   const int nC = J.nC, nWin = J.nWin, nPair = (nC - 1) / 2, nS = 1 + J.nA * nPair;
   auto wrap = [](int v) { return v < 0 ? v + W : (v >= W ? v - W : v); };
@@ -642,6 +674,7 @@ __global__ void __launch_bounds__(Cfg<N>::GC* Cfg<N>::T) k_pass_c(const JobDesc*
   const float2* tw = g_stw + stw_offset(N, EN);
   float2* s = sm + g * smem_line_elems(N, 1);
   const float2* twW = g_tw + tw_offset(W);
+  pdl_wait();
   const float2* row = J.O + (size_t)y * N;
   const float2 hn = J.On[y];
   float2 x[EN];  // element t + i*T of Z, in registers through the transform
@@ -718,33 +751,35 @@ static void launch_g(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, cu
   k_pass_g<N, ENA><<<dim3(maxA * maxPair, njobs), PA::T, 0, st>>>(d_jobs);
 }
 template <int N, int ENB, int CBB, bool CM>
-static int launch_b1_kind(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
+static int launch_b1_kind(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
   using PB = PassB1<N, ENB, CBB>;
   constexpr int CB = 2 * PB::CP;
   static bool attr = false, attr0 = false;
   int rc = grant_smem(k_pass_b1<N, ENB, CBB, CM>, PB::SMEM, attr);
   if (!rc) rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM0, attr0);
   if (rc) return rc;
-  k_pass_b1<N, ENB, CBB, CM><<<dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT, PB::SMEM, st>>>(d_jobs);
-  k_pass_b0<N, ENB, CBB, CM><<<dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM0, st>>>(d_jobs);
+  FSIM_CUDA(launch_pass(dep, k_pass_b0<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM0, st,
+                        d_jobs));
+  FSIM_CUDA(launch_pass(dep, k_pass_b1<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT,
+                        PB::SMEM, st, d_jobs));
   return FSIM_OK;
 }
 // masks: bit 0 launches the real-mask kind, bit 1 the complex-mask kind (measured OTFs)
 template <int N, int ENB, int CBB>
-static int launch_b1(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int masks, cudaStream_t st) {
+static int launch_b1(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int masks, cudaStream_t st) {
   int rc = FSIM_OK;
-  if (masks & 1) rc = launch_b1_kind<N, ENB, CBB, false>(d_jobs, njobs, maxA, maxPair, maxWin, st);
-  if (!rc && (masks & 2)) rc = launch_b1_kind<N, ENB, CBB, true>(d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (masks & 1) rc = launch_b1_kind<N, ENB, CBB, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && (masks & 2)) rc = launch_b1_kind<N, ENB, CBB, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
   return rc;
 }
 template <int N, int ENB, int CBB>
-static int launch_b2(const JobDesc* d_jobs, int njobs, cudaStream_t st) {
+static int launch_b2(bool dep, const JobDesc* d_jobs, int njobs, cudaStream_t st) {
   using PB = PassB2<N, ENB, CBB>;
   constexpr int CB = Cfg<N, ENB, CBB>::CB;
   static bool attr = false;
   int rc = grant_smem(k_pass_b2<N, ENB, CBB>, PB::SMEM, attr);
   if (rc) return rc;
-  k_pass_b2<N, ENB, CBB><<<dim3(N / CB + 1, njobs), PB::NT, PB::SMEM, st>>>(d_jobs);  // columns 0..N
+  FSIM_CUDA(launch_pass(dep, k_pass_b2<N, ENB, CBB>, dim3(N / CB + 1, njobs), PB::NT, PB::SMEM, st, d_jobs));  // 0..N
   return FSIM_OK;
 }
 
@@ -770,13 +805,17 @@ __host__ inline int size_slot(int n) {
 // (3*2^k sizes: 12, 24). The extremes (N <= 128, N >= 2048) have one variant.
 template <int N>
 int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip, int masks,
-                   cudaStream_t st) {
+                   bool alone, cudaStream_t st) {
   constexpr bool p3 = (N % 3 == 0);
   constexpr int E0 = p3 ? 12 : 8, E1 = p3 ? 24 : 16;
   constexpr bool single = (N <= 128 || N >= 2048);
   constexpr int CBX = N >= 2048 ? 2 : 4;
   const int k = size_slot(N);
   const int va = single ? 0 : g_var_a[k], vb1 = single ? 0 : g_var_b[k], vb2 = single ? 0 : g_var_b2[k];
+  // Passes as dependent launches while a batch is short: one 256^2 stack 46.8 -> 34.4 us, 8 x 512^2
+  // 186 -> 177, 16 x 512^2 (16k blocks of pass A) 336 -> 328, but 64 x 512^2 1183 -> 1195 us, and a batch of
+  // several size classes, whose waiting blocks take the room of another class's passes, 3% longer.
+  const bool dep = alone && (long long)(N / PassA<N, E0>::RB) * (maxA + 1) * njobs <= 64LL * ctx().num_sms;
   cudaEvent_t* ev = profile_events();
   if (ev) cudaEventRecord(ev[0], st);
   int rc = FSIM_OK;
@@ -789,31 +828,31 @@ int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int 
     else if constexpr (!single) launch_g<N, E1>(d_jobs, njobs, maxA, maxPair, st);
   }
   if constexpr (single) {
-    rc = launch_b1<N, E0, CBX>(d_jobs, njobs, maxA, maxPair, maxWin, masks, st);
+    rc = launch_b1<N, E0, CBX>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st);
   } else {
     switch (vb1) {
-      case 0: rc = launch_b1<N, E0, 4>(d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      case 1: rc = launch_b1<N, E0, 2>(d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      case 2: rc = launch_b1<N, E1, 4>(d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      default: rc = launch_b1<N, E1, 2>(d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
+      case 0: rc = launch_b1<N, E0, 4>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
+      case 1: rc = launch_b1<N, E0, 2>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
+      case 2: rc = launch_b1<N, E1, 4>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
+      default: rc = launch_b1<N, E1, 2>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
     }
   }
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[2], st);
   if constexpr (single) {
-    rc = launch_b2<N, E0, CBX>(d_jobs, njobs, st);
+    rc = launch_b2<N, E0, CBX>(dep, d_jobs, njobs, st);
   } else {
     switch (vb2) {
-      case 0: rc = launch_b2<N, E0, 4>(d_jobs, njobs, st); break;
-      case 1: rc = launch_b2<N, E0, 2>(d_jobs, njobs, st); break;
-      case 2: rc = launch_b2<N, E1, 4>(d_jobs, njobs, st); break;
-      default: rc = launch_b2<N, E1, 2>(d_jobs, njobs, st); break;
+      case 0: rc = launch_b2<N, E0, 4>(dep, d_jobs, njobs, st); break;
+      case 1: rc = launch_b2<N, E0, 2>(dep, d_jobs, njobs, st); break;
+      case 2: rc = launch_b2<N, E1, 4>(dep, d_jobs, njobs, st); break;
+      default: rc = launch_b2<N, E1, 2>(dep, d_jobs, njobs, st); break;
     }
   }
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[3], st);
   using PC = Cfg<N>;
-  k_pass_c<N><<<dim3(PC::W / PC::GC, njobs), PC::GC * PC::T, 0, st>>>(d_jobs);
+  FSIM_CUDA(launch_pass(dep, k_pass_c<N>, dim3(PC::W / PC::GC, njobs), PC::GC * PC::T, 0, st, d_jobs));
   if (scale_clip) k_scale_clip<<<dim3(2 * N, njobs), 256, 0, st>>>(d_jobs, 2 * N);
   if (ev) {
     cudaEventRecord(ev[4], st);
