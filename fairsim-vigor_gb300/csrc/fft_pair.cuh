@@ -141,6 +141,24 @@ __device__ __forceinline__ void dft8(cpair* v) {
   bfly_w8<INV, 3>(e3, o3, qq, v[3], v[7]);
 }
 template <bool INV>
+__device__ __forceinline__ void dft12(cpair* v) {
+  // 3 x 4 without twiddles: with n = 4 n1 + 3 n2 and k = k1 mod 3 = k2 mod 4 (both modulo 12),
+  // W12^{nk} = W3^{n1 k1} W4^{n2 k2}
+  cpair x[4][3];
+#pragma unroll
+  for (int n2 = 0; n2 < 4; n2++) {
+#pragma unroll
+    for (int n1 = 0; n1 < 3; n1++) x[n2][n1] = v[(4 * n1 + 3 * n2) % 12];
+    dft3<INV>(x[n2][0], x[n2][1], x[n2][2]);
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < 3; k1++) {
+    dft4<INV>(x[0][k1], x[1][k1], x[2][k1], x[3][k1]);
+#pragma unroll
+    for (int k2 = 0; k2 < 4; k2++) v[(4 * k1 + 9 * k2) % 12] = x[k2][k1];
+  }
+}
+template <bool INV>
 __device__ __forceinline__ void dft16(cpair* v) {
   // 4 x 4: sub-DFTs over m for v[q + 4m], twiddle W16^{q*k1}, then DFT4 over q.
   cpair x[4][4];
@@ -188,13 +206,14 @@ __device__ __forceinline__ void dft(cpair* v) {
   } else if constexpr (R == 3) dft3<INV>(v[0], v[1], v[2]);
   else if constexpr (R == 4) dft4<INV>(v[0], v[1], v[2], v[3]);
   else if constexpr (R == 8) dft8<INV>(v);
+  else if constexpr (R == 12) dft12<INV>(v);
   else if constexpr (R == 16) dft16<INV>(v);
 }
 
 // Exchange layouts: one element of padding per 8, or per 16 where a radix-16 stage writes with
 // stride 16; a stage's writes at stride R and its contiguous reads are then free of conflicts
-// for power-of-two lengths, and the position of element base + offset is layout(base) +
-// layout(offset) there (no carry into the padding), so that a thread's R accesses share one
+// at power-of-two strides, and the position of element base + offset is layout(base) +
+// layout(offset) where no carry reaches the padding, so that a thread's R accesses share one
 // address register.
 __host__ __device__ constexpr int pair_pad(int R) { return R == 16 ? 4 : 3; }
 template <int S>
@@ -204,10 +223,10 @@ __host__ __device__ constexpr int pair_elems(int L, int C) { return L * C + (L *
 template <int L, int T, int C, int R, int NS, bool INV, bool FIRST, bool LAST, int SIN>
 __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s, int c, int t, const float2* tw) {
   constexpr int E = L / T, NB = E / R, LR = L / R, SOUT = pair_pad(R);
-  constexpr bool P2 = is_pow2(L);
+  constexpr bool ADD_IN = is_pow2(L) || (LR * C) % (1 << SIN) == 0, ADD_OUT = is_pow2(NS * R);
   // stage table [r-1][k]: W^k, and W^2k, W^4k, W^8k where the radix has them; the other powers
   // by products (one rounding beyond the table's)
-  constexpr int NT = NS > 1 ? (R == 16 ? 4 : (R == 8 ? 3 : (R == 2 ? 1 : 2))) : 1;
+  constexpr int NT = NS > 1 ? (R > 8 ? 4 : (R >= 8 ? 3 : (R == 2 ? 1 : 2))) : 1;
   float2 tl[NB][NT];
   if constexpr (NS > 1) {
 #pragma unroll
@@ -216,7 +235,7 @@ __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s,
       tl[b][0] = tw[k];
       if constexpr (R >= 3) tl[b][1] = tw[NS + k];
       if constexpr (R >= 8) tl[b][2] = tw[3 * NS + k];
-      if constexpr (R == 16) tl[b][3] = tw[7 * NS + k];
+      if constexpr (R > 8) tl[b][3] = tw[7 * NS + k];
     }
   }
   cpair v[NB][R];
@@ -227,7 +246,7 @@ __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s,
     for (int r = 0; r < R; r++) {
       if constexpr (FIRST) v[b][r] = x[b + NB * r];
       else {
-        const ulonglong2 u = s[P2 ? lb + pair_lay<SIN>(r * LR * C) : pair_lay<SIN>(rb + r * LR * C)];
+        const ulonglong2 u = s[ADD_IN ? lb + pair_lay<SIN>(r * LR * C) : pair_lay<SIN>(rb + r * LR * C)];
         v[b][r] = cpair{u.x, u.y};
       }
     }
@@ -247,10 +266,10 @@ __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s,
 #pragma unroll
         for (int r = 5; r < 8; r++) w[r] = wmul(w[4], w[r - 4]);
       }
-      if constexpr (R == 16) {
+      if constexpr (R > 8) {
         w[8] = w_dup(tl[b][3]);
 #pragma unroll
-        for (int r = 9; r < 16; r++) w[r] = wmul(w[8], w[r - 8]);
+        for (int r = 9; r < R; r++) w[r] = wmul(w[8], w[r - 8]);
       }
 #pragma unroll
       for (int r = 1; r < R; r++) v[b][r] = INV ? cmulj(v[b][r], w[r]) : cmul(v[b][r], w[r]);
@@ -263,7 +282,7 @@ __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s,
       const int wb = ((j / NS) * NS * R + k) * C + c, lb = pair_lay<SOUT>(wb);
 #pragma unroll
       for (int r = 0; r < R; r++)
-        s[P2 ? lb + pair_lay<SOUT>(r * NS * C) : pair_lay<SOUT>(wb + r * NS * C)] =
+        s[ADD_OUT ? lb + pair_lay<SOUT>(r * NS * C) : pair_lay<SOUT>(wb + r * NS * C)] =
             make_ulonglong2(v[b][r].re, v[b][r].im);
     }
   }
@@ -271,7 +290,7 @@ __device__ __forceinline__ void fft_stage_pair(cpair (&x)[L / T], ulonglong2* s,
 }
 template <int L, int T, int C, bool INV, int NS, int SIN>
 __device__ __forceinline__ void fft_stages_pair(cpair (&x)[L / T], ulonglong2* s, int c, int t, const float2* tw) {
-  constexpr int R = pick_radix(L / NS, L / T);
+  constexpr int R = pick_radix_pair(L / NS, L / T);
   static_assert((L / NS) % R == 0 && (L / T) % R == 0, "bad radix plan");
   fft_stage_pair<L, T, C, R, NS, INV, NS == 1, NS * R == L, SIN>(x, s, c, t, tw);
   if constexpr (NS * R < L) fft_stages_pair<L, T, C, INV, NS * R, pair_pad(R)>(x, s, c, t, tw + (R - 1) * NS);
@@ -282,7 +301,7 @@ __device__ __forceinline__ void fft_stages_pair(cpair (&x)[L / T], ulonglong2* s
 template <int L, int T, int C, bool INV>
 __device__ __forceinline__ void line_fft_pair(cpair (&x)[L / T], ulonglong2* s, int c, int t, const float2* stw) {
   static_assert(supported_len(L) && plan_ok(L, T) && stw_ok(L, L / T), "no stage table for this plan");
-  fft_stages_pair<L, T, C, INV, 1, 3>(x, s, c, t, stw);
+  fft_stages_pair<L, T, C, INV, 1, 3>(x, s, c, t, stw + (pair_own_plan(L, L / T) ? stw_plan_len(L, L / T, false) : 0));
 }
 
 }  // namespace fsim

@@ -100,17 +100,17 @@ void fill_stage_twiddle_host(float2* h) {
       const int E = stw_e(e);
       if (!stw_ok(L, E)) continue;
       float2* t = h + stw_offset(L, E);
-      int rem = L, NS = 1, pos = 0;
-      while (rem > 1) {
-        const int R = pick_radix_fwd(rem, E);
-        for (int r = 1; r < R; r++)
-          for (int k = 0; k < NS; k++) {
-            double a = -2.0 * M_PI * (double)r * (double)k / ((double)NS * R);
-            t[pos++] = make_float2((float)std::cos(a), (float)std::sin(a));
-          }
-        NS *= R;
-        rem /= R;
-      }
+      for (int pair = 0; pair <= (int)pair_own_plan(L, E); pair++)
+        for (int rem = L, NS = 1; rem > 1;) {
+          const int R = pair ? pick_radix_pair(rem, E) : pick_radix_fwd(rem, E);
+          for (int r = 1; r < R; r++)
+            for (int k = 0; k < NS; k++) {
+              double a = -2.0 * M_PI * (double)r * (double)k / ((double)NS * R);
+              *t++ = make_float2((float)std::cos(a), (float)std::sin(a));
+            }
+          NS *= R;
+          rem /= R;
+        }
     }
   };
   for (int L = 16; L <= 8192; L *= 2) fill(L);

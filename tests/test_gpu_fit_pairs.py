@@ -78,3 +78,21 @@ def test_fft2d_pairs(fs, torch_cuda, w, h, batch, off, inverse):
         assert after[0] == edge[0] and after[1] == edge[1]  # nothing outside the planes is written
     else:
         assert after[1] == edge[1] and after[2] == edge[2]
+
+
+@pytest.mark.parametrize("w,h", [(48, 192), (96, 384), (192, 1536), (384, 768), (768, 96), (1536, 48)])
+@pytest.mark.parametrize("inverse", [0, 1])
+def test_fft2d_radix12_plans(fs, torch_cuda, w, h, inverse):
+    """Every 3*2^k plan that ends in a radix-12 stage, along rows and along columns; 1e-6 relative
+    L2 as above."""
+    torch = torch_cuda
+    N_ = fs.native
+    N_.init(0)
+    g = torch.Generator(device="cuda").manual_seed(w + h)
+    x = torch.randn(2, h, w, dtype=torch.complex64, device="cuda", generator=g)
+    f = torch.fft.ifft2 if inverse else torch.fft.fft2
+    ref = f(x.to(torch.complex128)).cpu().numpy()
+    torch.cuda.synchronize()
+    N_.check(N_.lib().fsim_fft2d_batch(C.c_void_p(x.data_ptr()), w, h, 2, inverse, None))
+    N_.check(N_.lib().fsim_sync())
+    assert rel_l2(x.cpu().numpy(), ref) < 1e-6
