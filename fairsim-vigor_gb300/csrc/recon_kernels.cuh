@@ -21,18 +21,6 @@
 #include "recon.cuh"
 #include "runtime.cuh"
 
-// Register budgets (registers per thread) of passes A, B1 and B2 at 8 elements per thread: two
-// lines of 8 complex values are 32 registers, a butterfly's operands and twiddles the rest.
-#ifndef FSIM_PA_REGS
-#define FSIM_PA_REGS 80
-#endif
-#ifndef FSIM_B1_REGS
-#define FSIM_B1_REGS 80
-#endif
-#ifndef FSIM_B2_REGS
-#define FSIM_B2_REGS 80
-#endif
-
 namespace fsim {
 
 // ---- launch configuration (variants picked per size by the autotuner) --------------------
@@ -68,10 +56,10 @@ __device__ __forceinline__ int paste_src(int X) {
 }
 
 // ---- pass A: rows ----------------------------------------------------------------------------
-// Blocks per SM for regs8 registers per thread at 8 elements, 128 at 12 or 16, 255 beyond
-// (line pairs hold 4 registers per element; a partial warp takes a whole one's registers).
+// Blocks per SM for regs8 registers per thread at 8 elements, 128 at 12, 255 beyond (a line pair
+// holds 4 registers per element; a partial warp takes a whole one's registers).
 __host__ __device__ constexpr int pair_min_blocks(int threads, int EN, int regs8) {
-  const int r = EN <= 8 ? regs8 : (EN <= 16 ? 128 : 255), n = threads < 32 ? 32 : threads;
+  const int r = EN <= 8 ? regs8 : (EN <= 12 ? 128 : 255), n = threads < 32 ? 32 : threads;
   return 65536 / (n * r) > 0 ? (65536 / (n * r) < 32 ? 65536 / (n * r) : 32) : 1;
 }
 // Raw pixels of the rows at `row` and the row below (frame offset fo) with the background clip:
@@ -119,8 +107,7 @@ __device__ __forceinline__ void damp_rows(const JobDesc& J, size_t row, int t, c
 }
 
 // A group of T threads transforms two adjacent rows as one line pair; groups are joined to
-// blocks of at least 64 threads. Dynamic shared memory per group: the exchange buffer of the
-// pair, then a stash of one pair whose entries only their own thread uses.
+// blocks of at least 64 threads. Dynamic shared memory: the exchange buffer of each group's pair.
 template <int N, int ENV>
 struct PassA {
   static constexpr int T = Cfg<N, ENV>::T, EN = Cfg<N, ENV>::EN;
@@ -128,15 +115,14 @@ struct PassA {
   static constexpr int NT = G * T;
   static constexpr int RB = 2 * G;  // rows per block
   static constexpr int XS = pair_elems(N, 1);
-  static constexpr int GS = XS + N;  // shared-memory elements per group
-  static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)G * GS;
-  // Frames whose pixels are in flight at once while a thread mixes them. Three frames take 96
-  // registers where one takes 80, but blocks of 64 threads lose little residence by it: 64 x 512^2
-  // 491 -> 473 us. Larger blocks lose more (2048^2: two blocks per SM instead of three, the whole
-  // reconstruction 464 -> 497 us; 8 x 1024^2 750 -> 756), and 12 elements per thread leave no room
-  // (8 x 768^2 594 -> 596).
-  static constexpr int F = (NT <= 64 && EN <= 8) ? 3 : 1;
-  static constexpr int MINB = pair_min_blocks(NT, EN, F > 1 ? 96 : FSIM_PA_REGS);
+  static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)G * XS;
+  // Frames whose pixels are in flight at once while a thread mixes them, and the registers that
+  // takes: with 64 threads 3 (96 registers) against 1 (80) is 447 us against 451 for 64 x 512^2, with
+  // 128 threads 531 against 565 for 16 x 1024^2; at 256 threads 96 registers leave two blocks per
+  // SM instead of three (a 2048^2 3x5 stack: 238 us, 201 with one frame, 195 with two). 12
+  // elements per thread leave no room for more than one.
+  static constexpr int F = EN > 8 ? 1 : (NT <= 128 ? 3 : 2);
+  static constexpr int MINB = pair_min_blocks(NT, EN, F == 3 ? 96 : 80);
   static_assert(N % RB == 0, "whole blocks of rows");
 };
 
@@ -153,7 +139,7 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   __shared__ JobDesc J;
   __shared__ float2 coef[FSIM_MAX_DIRS * FSIM_MAX_PHASES];
   extern __shared__ ulonglong2 smp[];
-  ulonglong2* s = smp + g * PA::GS;
+  ulonglong2* s = smp + g * PA::XS;
   const float2* twN = g_stw + stw_offset(N, EN);  // stage table, read through L1
   const float2* twW = g_tw + tw_offset(W);
   pdl_trigger();
@@ -246,12 +232,15 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   //   (V_neg + V+) / 2 = Ty Tx z - Qy Qx z.
   // So this pass drops the Nyquist bin (s(N/2) = 0) and keeps its value per row (D); the column
   // pass puts -Qy Qx z back as the column's own Nyquist value.
-  ulonglong2* stash = s + PA::XS + t;  // entries i * T: this thread's own
+  // z holds the mixed rows, then E: in shared memory (8 or 12 more 16-byte elements per thread each
+  // way, twice) the shared-memory pipe, which bounds this pass, took 474 us per 64 x 512^2 in place of
+  // 447, and 374 us per 16 x 768^2 in place of 333.
+  cpair z[EN];
   for (int b = 1; b <= nPair; b++) {
     const int cn = 2 * b - 1;
     mix(a * nP, nP, coef + cn * nP);
 #pragma unroll
-    for (int i = 0; i < EN; i++) stash[i * T] = make_ulonglong2(x[i].re, x[i].im);
+    for (int i = 0; i < EN; i++) z[i] = x[i];
     const float2* re = J.ramps + (size_t)(a * nC + cn) * 2 * W;
     const float2* ro = re + N;
     // even samples times the even-sample ramp, FFT: E (changes places with the mixed rows)
@@ -260,9 +249,9 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
     line_fft_pair<N, T, 1, false>(x, s, 0, t, twN);
 #pragma unroll
     for (int i = 0; i < EN; i++) {
-      const ulonglong2 z = stash[i * T];
-      stash[i * T] = make_ulonglong2(x[i].re, x[i].im);
-      x[i] = cpair{z.x, z.y};
+      const cpair e = x[i];
+      x[i] = z[i];
+      z[i] = e;
     }
     line_fft_pair<N, T, 1, false>(x, s, 0, t, twN);  // Z = FFT_N(z)
     if (t == (N / 2) % T) {
@@ -286,8 +275,6 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
     float2* I = J.I + (size_t)(1 + a * nPair + (b - 1)) * nWin * N;  // slot of (a, b)
 #pragma unroll
     for (int i = 0; i < EN; i++) {
-      const ulonglong2 u = stash[i * T];
-      const cpair e = cpair{u.x, u.y};
       int xl = t + i * T - Xs;
       if (xl < 0) xl += W;
       if (xl >= N) xl -= N;
@@ -295,8 +282,8 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
         int X = Xs + xl;
         if (X >= W) X -= W;
         const cpair o = cmul(x[i], w_dup(__ldg(twW + X)));
-        put(I, xl, cadd(e, o));
-        if (xl + N < nWin) put(I, xl + N, csub(e, o));
+        put(I, xl, cadd(z[i], o));
+        if (xl + N < nWin) put(I, xl + N, csub(z[i], o));
       }
     }
   }
@@ -368,15 +355,17 @@ __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __rest
 // because mask_pos(X, Y) = mask_neg(-X, -Y). With the masks and the Nyquist terms applied here,
 // where the column is in registers, pass B2 only adds windows (it took 0.358 ms per 64 datasets
 // of 512^2 3x3 while it read neg and pos masks and formed the Nyquist terms per pixel).
-// Adjacent columns form a line pair: CB/2 pairs of T threads per block, with pass A's exchange
-// buffer and stash.
+// Adjacent columns form a line pair: CB/2 pairs of T threads per block. Each thread keeps the
+// column and then E in registers, as pass A does (in shared memory 395 us per 64 x 512^2 in place
+// of 367); the transforms' operands beside them fit 80 registers without spills worth their time
+// (72: 396 us, 96: 382).
 template <int N, int ENV, int CBV>
 struct PassB1 {
   using P = Cfg<N, ENV, CBV>;
   static constexpr int CP = P::CB / 2, NT = CP * P::T;
   static constexpr int XS = pair_elems(N, CP);
-  static constexpr size_t SMEM = sizeof(ulonglong2) * ((size_t)XS + N * CP), SMEM0 = sizeof(ulonglong2) * (size_t)XS;
-  static constexpr int MINB = pair_min_blocks(NT, P::EN, FSIM_B1_REGS);
+  static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)XS;
+  static constexpr int MINB = pair_min_blocks(NT, P::EN, 80);
 };
 // Row yl of window columns xl and xl + 1 of a component (col: the position of its first row in
 // the component-by-component window layout), times their masks, to Tw.
@@ -455,7 +444,7 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   __shared__ float2 part[(NT + 31) / 32];
   extern __shared__ ulonglong2 smp[];
   ulonglong2* s = smp;
-  ulonglong2* stash = smp + PB::XS + lt;  // entries i * NT: this thread's own
+  cpair z[EN];
   const float2* twN = g_stw + stw_offset(N, EN);
   const float2* twW = g_tw + tw_offset(W);
   load_job(&J, jobs + blockIdx.z, lt, NT);
@@ -491,15 +480,15 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   // even samples times the even-sample ramp, FFT: E (changes places with the column)
 #pragma unroll
   for (int i = 0; i < EN; i++) {
-    stash[i * NT] = make_ulonglong2(x[i].re, x[i].im);
+    z[i] = x[i];
     x[i] = cmul(x[i], w_dup(__ldg(re + t + i * T)));
   }
   line_fft_pair<N, T, CP, false>(x, s, lane, t, twN);
 #pragma unroll
   for (int i = 0; i < EN; i++) {
-    const ulonglong2 z = stash[i * NT];
-    stash[i * NT] = make_ulonglong2(x[i].re, x[i].im);
-    x[i] = cpair{z.x, z.y};
+    const cpair e = x[i];
+    x[i] = z[i];
+    z[i] = e;
   }
   line_fft_pair<N, T, CP, false>(x, s, lane, t, twN);  // Z along y
   const float2* nx = J.nyq + (size_t)ab * 2 * nWin;  // Qx over the window columns, Qy over its rows
@@ -539,8 +528,6 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   };
 #pragma unroll
   for (int i = 0; i < EN; i++) {
-    const ulonglong2 u = stash[i * NT];
-    const cpair e = cpair{u.x, u.y};
     int yl = t + i * T - Ys;
     if (yl < 0) yl += W;
     if (yl >= N) yl -= N;
@@ -548,8 +535,8 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
       int Y = Ys + yl;
       if (Y >= W) Y -= W;
       const cpair o = cmul(x[i], w_dup(__ldg(twW + Y)));
-      finish(yl, cadd(e, o));
-      if (yl + N < nWin) finish(yl + N, csub(e, o));
+      finish(yl, cadd(z[i], o));
+      if (yl + N < nWin) finish(yl + N, csub(z[i], o));
     }
   }
   pdl_wait();
@@ -571,7 +558,7 @@ struct PassB2 {
   using P = Cfg<N, ENV, CBV>;
   static constexpr int NT = P::CB * P::T;
   static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)pair_elems(N, P::CB);
-  static constexpr int MINB = pair_min_blocks(NT, P::EN, FSIM_B2_REGS);
+  static constexpr int MINB = pair_min_blocks(NT, P::EN, 80);
 };
 template <int N, int ENV, int CBV>
 __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::MINB)
@@ -756,9 +743,9 @@ static int launch_b1_kind(bool dep, const JobDesc* d_jobs, int njobs, int maxA, 
   constexpr int CB = 2 * PB::CP;
   static bool attr = false, attr0 = false;
   int rc = grant_smem(k_pass_b1<N, ENB, CBB, CM>, PB::SMEM, attr);
-  if (!rc) rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM0, attr0);
+  if (!rc) rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM, attr0);
   if (rc) return rc;
-  FSIM_CUDA(launch_pass(dep, k_pass_b0<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM0, st,
+  FSIM_CUDA(launch_pass(dep, k_pass_b0<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM, st,
                         d_jobs));
   FSIM_CUDA(launch_pass(dep, k_pass_b1<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT,
                         PB::SMEM, st, d_jobs));
