@@ -1,6 +1,6 @@
 // Fused, batched 2D SIM reconstruction: SimAlgorithm.runReconstruction
 // (S/SimAlgorithm.java:268-582; Wiener filter style, OTF applied after a Fourier shift on
-// the 2w x 2w grid) in three passes over HBM instead of ~40 vector ops.
+// the 2w x 2w grid) in four passes over HBM instead of ~40 vector ops.
 //
 // The reference's per-component chain, with W = 2N,
 //   sep_c = sum_p M[c][p] FFT_N(raw_p);  V_c = FFT_W(ramp_c * iFFT_W(paste(sep_c)));
@@ -12,9 +12,10 @@
 //      x, paste, and for shifted components the x half of the shift
 //      (iFFT_W, ramp_x, FFT_W) -> only the columns inside each component's OTF support
 //      window are written (the OTF zeroes everything else);
-//   B  (columns, per dataset x 4-column quad): FFT_N along y, paste, y half of the shift,
-//      times the exact conj(OTF) mask, accumulate all components, times wiener*apo,
-//      iFFT_W along y;
+//   B1 (columns of each component's window): FFT_N along y, paste, y half of the shift, times
+//      the exact conj(OTF) mask;
+//   B2 (columns 0..N of the output spectrum, whose other half is its mirror image): the masked
+//      windows summed, times wiener*apo, iFFT_W along y;
 //   C  (rows,    per output row): iFFT_W along x, real part, 1/W^2.
 // Shift phases use exact per-axis ramp tables; OTF masks and the Wiener*apo filter are
 // resident per plan, built with the reference's floor-indexed OTF lookup (table positions in

@@ -56,10 +56,10 @@ __device__ __forceinline__ int paste_src(int X) {
 }
 
 // ---- pass A: rows ----------------------------------------------------------------------------
-// Blocks per SM for regs8 registers per thread at 8 elements, 128 at 12, 255 beyond (a line pair
+// Blocks per SM for regs8 registers per thread at 8 elements, 128 at 12 or 16, 255 beyond (a line pair
 // holds 4 registers per element; a partial warp takes a whole one's registers).
 __host__ __device__ constexpr int pair_min_blocks(int threads, int EN, int regs8) {
-  const int r = EN <= 8 ? regs8 : (EN <= 12 ? 128 : 255), n = threads < 32 ? 32 : threads;
+  const int r = EN <= 8 ? regs8 : (EN <= 16 ? 128 : 255), n = threads < 32 ? 32 : threads;
   return 65536 / (n * r) > 0 ? (65536 / (n * r) < 32 ? 65536 / (n * r) : 32) : 1;
 }
 // Raw pixels of the rows at `row` and the row below (frame offset fo) with the background clip:
