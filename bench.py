@@ -173,14 +173,13 @@ def run_reference(args):
 
 
 # DRAM bytes (read + write) per dataset of each pass at 512^2 3x3, from single-kernel ncu
-# captures (dram__bytes_read.sum + dram__bytes_write.sum; `ncu --set full -k regex:<pass>
-# -s 2 -c 1` of `bench.py --batch 16 --steps 3 --warmup 3 --no-extras`, raw 151 MB, larger than
-# L2); per-launch traffic = this x the batch size. G+B1 counts B1 (G moves 0.04 MB). Pass C is
+# captures (dram__bytes_read.sum + dram__bytes_write.sum; `ncu --set full -k regex:k_pass_` of a
+# batch of 16, raw 151 MB, larger than L2); per-launch traffic = this x the batch size. Pass C is
 # left out: at batch 16 its input, the Hermitian halves pass B2 has just written (67 MB), is
 # still in L2, so the capture does not show its DRAM traffic at batch 64.
-TRAFFIC_PER_DATASET = {"k_pass_a<512>": 15.99e6, "k_pass_g+k_pass_b1<512>": 11.21e6, "k_pass_b2<512>": 14.20e6,
+TRAFFIC_PER_DATASET = {"k_pass_a<512>": 15.33e6, "k_pass_b0+k_pass_b1<512>": 10.81e6, "k_pass_b2<512>": 9.26e6,
                        "k_pass_c<512>": None}
-PASS_NAMES = ["k_pass_a<512>", "k_pass_g+k_pass_b1<512>", "k_pass_b2<512>", "k_pass_c<512>"]
+PASS_NAMES = ["k_pass_a<512>", "k_pass_b0+k_pass_b1<512>", "k_pass_b2<512>", "k_pass_c<512>"]
 
 
 def pass_bytes(n=N, n_dirs=NA, n_phases=NP, n_bands=NB, na=1.4, lam=525.0, pxl=0.08):
@@ -188,13 +187,11 @@ def pass_bytes(n=N, n_dirs=NA, n_phases=NP, n_bands=NB, na=1.4, lam=525.0, pxl=0
     written once):
       A      raw frames in; row-transformed OTF-support windows I out (band 0 of all angles
              summed, once; each angle's pair neg components), plus one Nyquist term per row (D)
-      G+B1   D in, one column per angle and pair out (G); I in, the column-transformed windows
-             Tw (band 0, neg of every pair) and one Nyquist term per neg column (Dy) out
-      B2     over the Hermitian half's columns 0..N: Tw (each neg window column once: at X for
-             the neg component, at -X for the pos one; band 0 half a window), the OTF masks
-             (a pair's neg and pos windows are mirror images, so together they cover one
-             window's columns; band 0 half a window), the Wiener x apodization table, G, Dy
-             in; the W x (N+1) Hermitian half out
+      B0+B1  I and D in, the OTF masks (band 0, neg of every pair), the masked column-transformed
+             windows Tw out
+      B2     over the Hermitian half's columns 0..N: Tw (each neg window column once: at X, or
+             at -X for its mirror image; band 0 half a window) and the Wiener x apodization
+             table in; the W x (N+1) Hermitian half out
       C      the Hermitian half in, the W x W image out"""
     npair = n_bands - 1
     W = 2 * n
@@ -202,14 +199,12 @@ def pass_bytes(n=N, n_dirs=NA, n_phases=NP, n_bands=NB, na=1.4, lam=525.0, pxl=0
     nwin = min(W, ((2 * int(np.ceil(R)) + 6) // 4) * 4 + 4)
     I = (1 + n_dirs * npair) * nwin * n * 8  # band 0 summed over the angles in pass A
     D = n_dirs * npair * n * 8
-    G = n_dirs * npair * nwin * 8
     Tw = (1 + n_dirs * npair) * nwin * nwin * 8
-    Dy = n_dirs * npair * nwin * 8
-    masks = (0.5 + n_dirs * npair) * nwin * nwin * 4
+    masks = (1 + n_dirs * npair) * nwin * nwin * 4
     OH = W * (n + 1) * 8
     a = n_dirs * n_phases * n * n * 4 + I + D
-    b1 = D + G + I + Tw + Dy
-    b2 = (0.5 + n_dirs * npair) * nwin * nwin * 8 + masks + (n + 1) * W * 4 + G + Dy + OH
+    b1 = D + I + masks + Tw
+    b2 = (0.5 + n_dirs * npair) * nwin * nwin * 8 + (n + 1) * W * 4 + OH
     c = OH + W * W * 4
     return [a, b1, b2, c]
 
