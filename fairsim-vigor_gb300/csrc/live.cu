@@ -28,7 +28,7 @@
 // The OTF also zeroes every column beyond its support: only a window of columns leaves LA.
 // Rows (LA, LC) and columns (LB, LD) are transformed two at a time (fft_pair.cuh). Bound by the
 // shared-memory pipe and instruction issue of 11.6k transforms of length N per 512^2 3x3 stack (26k
-// with every component and the full grid): 64 stacks in 1087 us on GB300, 2382 us before; one
+// with every component and the full grid): 64 stacks in 1069 us on GB300, 2382 us before; one
 // stack 62.6 us, 109 before.
 #include <cmath>
 #include <vector>
@@ -54,13 +54,13 @@ struct LCfg {
   static constexpr int G = T >= 64 ? 1 : 64 / T;    // row pairs per block, passes LA and LC
   static constexpr int CP = 2;                      // column pairs per block, pass LB
   static constexpr int CD = N >= 2048 ? 2 : 4;      // column pairs per block, pass LD
-  // Registers per thread at 8 elements: 80, but 96 in pass LA, which keeps two frames' pixels in
+  // Registers per thread at 8 elements: 64 in passes LB and LD (against 80, 64 x 512^2: 217 -> 212 and
+  // 129 -> 125 us; 16 x 1024^2: 305 -> 301 and 186 -> 152), 96 in pass LA, which keeps two frames' pixels in
   // flight while it mixes (64 x 512^2: 361 -> 318 us; three frames 342), and 128 in pass LC, which
   // loads the next contribution during a transform (474 -> 436 us; 531 at 80, where it spills).
-  static constexpr int R = E <= 8 ? 80 : 128;
   static constexpr int RA = 96, RC = 128, F = 2;
-  static constexpr int blocks(int threads, int regs8 = 80) {
-    const int n = threads < 32 ? 32 : threads, b = 65536 / (n * (E <= 8 ? regs8 : R));
+  static constexpr int blocks(int threads, int regs8 = 64) {
+    const int n = threads < 32 ? 32 : threads, b = 65536 / (n * (E <= 8 ? regs8 : 128));
     return b < 1 ? 1 : (b > 32 ? 32 : b);
   }
   static constexpr int XS = pair_elems(N, 1);       // exchange buffer of one pair

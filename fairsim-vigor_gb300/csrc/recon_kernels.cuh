@@ -558,7 +558,9 @@ struct PassB2 {
   using P = Cfg<N, ENV, CBV>;
   static constexpr int NT = P::CB * P::T;
   static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)pair_elems(N, P::CB);
-  static constexpr int MINB = pair_min_blocks(NT, P::EN, 80);
+  // 80 registers hold the sums without spills (64 x 512^2: 207 us, 240 at 64); at 512 threads they leave
+  // one block per SM, and 64 leave two (a 2048^2 3x5 stack: 94 -> 86 us)
+  static constexpr int MINB = pair_min_blocks(NT, P::EN, NT >= 512 ? 64 : 80);
 };
 template <int N, int ENV, int CBV>
 __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::MINB)
