@@ -477,6 +477,7 @@ int Plan::build_live(cudaStream_t st) {
   const int N = prm.w, W = 2 * N, nA = prm.nr_dirs, nP = prm.nr_phases, nC = 2 * prm.nr_bands - 1;
   OtfTable ht;
   build_otf_table(&prm, &ht);
+  const int old_nwin = nwin;
   // window of spectrum columns inside the OTF support (all columns when it is wider), from Xs
   plan_window(&prm, ht.cutoff / ht.vec_cpm, &nwin);
   if (nwin > N) nwin = N;
@@ -528,12 +529,15 @@ int Plan::build_live(cudaStream_t st) {
   size_t o_wa = o_mask + al((size_t)N * N * sizeof(float));
   size_t o_apo = o_wa + al((size_t)W * W * sizeof(float));
   size_t total = o_apo + al((size_t)(N + 1) * (N + 1) * sizeof(float));
+  const void* old_dev = dev;
   if (total > dev_bytes) {
     if (dev) cudaFree(dev);
     dev = nullptr;
+    dev_bytes = 0;
     FSIM_CUDA(fsim::dev_alloc(&dev, total));
     dev_bytes = total;
   }
+  if (old_dev != dev || old_nwin != nwin) layout->fetch_add(1);
   char* b = (char*)dev;
   d_coef = (float2*)(b + o_coef);
   d_ramps = (float2*)(b + o_ramp);
@@ -604,6 +608,7 @@ void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, cha
   j.clip_max = nullptr;
   j.clip = 0;
   j.cmask = 0;
+  j.edge = nullptr;
   j.fwf = nullptr;
   j.wff = nullptr;
   j.Wf = nullptr;

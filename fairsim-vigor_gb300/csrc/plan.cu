@@ -11,11 +11,18 @@
 
 struct fsim_plan : fsim::Plan {};
 
-// A fixed batch recorded as a CUDA graph (fsim_batch_graph_*).
+// A fixed batch recorded as a CUDA graph (fsim_batch_graph_*). The record holds what the plans were
+// when it was made; a plan updated since to other tables, another window or another
+// kind (Plan::layout) has the batch recorded again at the next launch.
 struct fsim_batch_graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaStream_t aux[3] = {};
+  cudaStream_t st = nullptr, aux[3] = {};
+  std::vector<fsim_job> jobs;
+  void* ws = nullptr;
+  size_t ws_bytes = 0;
+  std::vector<std::pair<std::shared_ptr<std::atomic<unsigned>>, unsigned>> layouts;  // of the jobs' plans
+  std::mutex mu;
   int n_jobs = 0;
   int kernels = 0;
 };
@@ -147,15 +154,15 @@ int recon_batch(const fsim_job* jobs, int n, void* ws, size_t ws_bytes, cudaStre
     // largest classes sort last; the first class stays on st, the rest spread over aux
     cudaStream_t s = (nfork > 0 && g > 0) ? aux[(g - 1) % nfork] : st;
     bool scale_clip = false;
-    int masks = 0;
+    int kinds = 0;
     for (int i = k; i < e; i++) {
       const Plan* pi = static_cast<const Plan*>(jobs[order[i]].plan);
       scale_clip = scale_clip || pi->clip_scale == 2;
-      masks |= otf_measured(&pi->prm) ? 2 : 1;
+      kinds |= pi->kind();
     }
     rc = (p0->path == FSIM_PATH_LIVE)
              ? launch_live_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, s)
-             : launch_offline_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, scale_clip, masks, nfork == 0, s);
+             : launch_offline_size(p0->prm.w, d_table + k, e - k, maxA, maxPair, maxWin, scale_clip, kinds, nfork == 0, s);
     if (rc == FSIM_OK && p0->path == FSIM_PATH_OFFLINE) {
       bool wf = false;
       for (int i = k; i < e; i++) wf = wf || jobs[order[i]].widefield || jobs[order[i]].filtered_widefield;
@@ -191,6 +198,75 @@ static cudaEvent_t g_prof_ev[8];
 static int g_prof_n = 0;
 cudaEvent_t* profile_events() { return g_prof_on ? g_prof_ev : nullptr; }
 void profile_mark(int n_passes) { g_prof_n = n_passes; }
+
+// Records the batch of g's jobs and instantiates it in place of the former record, which stays if
+// this fails.
+static int record_graph(fsim_batch_graph* g) {
+  // the job table is a kernel parameter of the captured put launch: every replay writes it
+  // to the workspace head before the passes, so the graph does not depend on what else used
+  // the workspace in between
+  std::vector<JobDesc> table(g->n_jobs);
+  const bool prof = g_prof_on;
+  g_prof_on = false;  // profiling events are not recorded inside a graph
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  int rc = FSIM_OK;
+  cudaError_t e = cudaStreamBeginCapture(g->st, cudaStreamCaptureModeRelaxed);
+  if (e != cudaSuccess) {
+    set_error("batch_graph: begin capture: %s", cudaGetErrorString(e));
+    rc = FSIM_ECUDA;
+  } else {
+    rc = recon_batch(g->jobs.data(), g->n_jobs, g->ws, g->ws_bytes, g->st, table.data(), true, g->aux, FSIM_AUX_STREAMS);
+    e = cudaStreamEndCapture(g->st, &graph);
+    if (rc == FSIM_OK && e != cudaSuccess) {
+      set_error("batch_graph: end capture: %s", cudaGetErrorString(e));
+      rc = FSIM_ECUDA;
+    }
+  }
+  g_prof_on = prof;
+  if (rc == FSIM_OK) {
+    e = cudaGraphInstantiate(&exec, graph, 0);
+    if (e != cudaSuccess) {
+      set_error("batch_graph: instantiate: %s", cudaGetErrorString(e));
+      rc = FSIM_ECUDA;
+    }
+  }
+  if (rc != FSIM_OK) {
+    if (graph) cudaGraphDestroy(graph);
+    cudaGetLastError();
+    return rc;
+  }
+  size_t nn = 0;
+  cudaGraphGetNodes(graph, nullptr, &nn);
+  std::vector<cudaGraphNode_t> nodes(nn);
+  if (nn) cudaGraphGetNodes(graph, nodes.data(), &nn);
+  g->kernels = 0;
+  for (auto nd : nodes) {
+    cudaGraphNodeType t;
+    if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) g->kernels++;
+  }
+  if (g->exec) {
+    cudaDeviceSynchronize();  // launches of the former record may be in flight
+    cudaGraphExecDestroy(g->exec);
+    cudaGraphDestroy(g->graph);
+  }
+  g->graph = graph;
+  g->exec = exec;
+  g->layouts.clear();
+  for (const fsim_job& j : g->jobs) {
+    const auto& l = static_cast<const Plan*>(j.plan)->layout;
+    g->layouts.emplace_back(l, l->load());
+  }
+  return FSIM_OK;
+}
+static void free_graph(fsim_batch_graph* g) {
+  if (g->exec) cudaGraphExecDestroy(g->exec);
+  if (g->graph) cudaGraphDestroy(g->graph);
+  if (g->st) cudaStreamDestroy(g->st);
+  for (auto a : g->aux)
+    if (a) cudaStreamDestroy(a);
+  delete g;
+}
 
 size_t batch_workspace_bytes(const Plan* const* plans, int n) {
   size_t need = align256(sizeof(JobDesc) * n);
@@ -346,62 +422,16 @@ int fsim_batch_graph_create(fsim_batch_graph** out, const fsim_job* jobs, int n_
   FSIM_REQUIRE(cs == cudaStreamCaptureStatusNone, FSIM_EINVAL, "batch_graph_create: stream is already capturing");
   fsim_batch_graph* g = new fsim_batch_graph();
   g->n_jobs = n_jobs;
-  auto fail = [&](int rc) {
-    for (auto a : g->aux)
-      if (a) cudaStreamDestroy(a);
-    delete g;
+  g->jobs.assign(jobs, jobs + n_jobs);
+  g->ws = workspace;
+  g->ws_bytes = workspace_bytes;
+  bool ok = cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking) == cudaSuccess;
+  for (auto& a : g->aux) ok = ok && cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking) == cudaSuccess;
+  int rc = ok ? record_graph(g) : FSIM_ECUDA;
+  if (!ok) set_error("batch_graph_create: stream creation failed");
+  if (rc) {
+    free_graph(g);
     return rc;
-  };
-  // the job table is a kernel parameter of the captured put launch: every replay writes it
-  // to the workspace head before the passes, so the graph does not depend on what else used
-  // the workspace in between
-  std::vector<JobDesc> table(n_jobs);
-  for (auto& a : g->aux)
-    if (cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking) != cudaSuccess) {
-      set_error("batch_graph_create: stream creation failed");
-      return fail(FSIM_ECUDA);
-    }
-  const bool prof = g_prof_on;
-  g_prof_on = false;  // profiling events are not recorded inside a graph
-  cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
-  int rc = FSIM_OK;
-  if (e != cudaSuccess) {
-    set_error("batch_graph_create: begin capture: %s", cudaGetErrorString(e));
-    rc = FSIM_ECUDA;
-  } else {
-    rc = recon_batch(jobs, n_jobs, workspace, workspace_bytes, st, table.data(), true, g->aux,
-                     FSIM_AUX_STREAMS);
-    cudaGraph_t graph = nullptr;
-    e = cudaStreamEndCapture(st, &graph);
-    if (rc == FSIM_OK && e != cudaSuccess) {
-      set_error("batch_graph_create: end capture: %s", cudaGetErrorString(e));
-      rc = FSIM_ECUDA;
-    }
-    g->graph = graph;
-  }
-  g_prof_on = prof;
-  if (rc == FSIM_OK) {
-    e = cudaGraphInstantiate(&g->exec, g->graph, 0);
-    if (e != cudaSuccess) {
-      set_error("batch_graph_create: instantiate: %s", cudaGetErrorString(e));
-      rc = FSIM_ECUDA;
-    }
-  }
-  if (rc == FSIM_OK) {
-    size_t nn = 0;
-    cudaGraphGetNodes(g->graph, nullptr, &nn);
-    std::vector<cudaGraphNode_t> nodes(nn);
-    if (nn) cudaGraphGetNodes(g->graph, nodes.data(), &nn);
-    for (auto nd : nodes) {
-      cudaGraphNodeType t;
-      if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) g->kernels++;
-    }
-  }
-  if (rc != FSIM_OK) {
-    if (g->exec) cudaGraphExecDestroy(g->exec);
-    if (g->graph) cudaGraphDestroy(g->graph);
-    cudaGetLastError();
-    return fail(rc);
   }
   *out = g;
   return FSIM_OK;
@@ -410,6 +440,13 @@ int fsim_batch_graph_create(fsim_batch_graph** out, const fsim_job* jobs, int n_
 int fsim_batch_graph_launch(fsim_batch_graph* g, void* stream) {
   FSIM_REQUIRE(g && g->exec, FSIM_EINVAL, "batch_graph_launch: null graph");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+  std::lock_guard<std::mutex> lock(g->mu);
+  for (const auto& l : g->layouts)
+    if (l.first->load(std::memory_order_relaxed) != l.second) {
+      int rc = record_graph(g);
+      if (rc) return rc;
+      break;
+    }
   FSIM_CUDA(cudaGraphLaunch(g->exec, st));
   return FSIM_OK;
 }
@@ -424,11 +461,7 @@ int fsim_batch_graph_info(const fsim_batch_graph* g, int* n_jobs, int* n_kernels
 int fsim_batch_graph_destroy(fsim_batch_graph* g) {
   if (!g) return FSIM_OK;
   cudaDeviceSynchronize();
-  if (g->exec) cudaGraphExecDestroy(g->exec);
-  if (g->graph) cudaGraphDestroy(g->graph);
-  for (auto a : g->aux)
-    if (a) cudaStreamDestroy(a);
-  delete g;
+  free_graph(g);
   return FSIM_OK;
 }
 

@@ -60,24 +60,56 @@ __global__ void k_build_mask(float* __restrict__ mask, int W, int nWin, int Xs, 
 
 // 1/(sum |OTF|^2 + w^2) * apo, quad layout [X/4][Y][X%4], for the columns X < ncols; the
 // apodization from its octant table apo (W/2 + 1 entries per row)
-__global__ void k_build_wa(float* __restrict__ wa, int ncols, int W, const OtfTable* __restrict__ t, ShiftSet shifts,
-                           FShiftSet fsh, int use_att, float wp, const float* __restrict__ apo) {
-  const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y;
-  if (X >= ncols) return;
+struct WaArgs {
+  const OtfTable* otf;
+  ShiftSet shifts;
+  FShiftSet fsh;
+  int use_att;
+  float wp;
+  const float* apo;
+};
+__device__ __forceinline__ float wa_at(const WaArgs& A, int X, int Y, int W) {
   const int xh = freq_x(X, W), yh = freq_y(Y, W);
   float acc = 0.f;
-  for (int d = 0; d < shifts.n_dirs; d++)
-    for (int b = 0; b < shifts.n_bands; b++) {
-      const double kx = shifts.px[d] * b, ky = shifts.py[d] * b;
-      const FShift k = fsh.k[d][b];
-      const float v1 = wiener_term(*t, b, xh, yh, k, kx, ky, use_att != 0);
-      const float v2 = wiener_term(*t, b, xh, yh, fshift_neg(k), -kx, -ky, use_att != 0);
+  for (int d = 0; d < A.shifts.n_dirs; d++)
+    for (int b = 0; b < A.shifts.n_bands; b++) {
+      const double kx = A.shifts.px[d] * b, ky = A.shifts.py[d] * b;
+      const FShift k = A.fsh.k[d][b];
+      const float v1 = wiener_term(*A.otf, b, xh, yh, k, kx, ky, A.use_att != 0);
+      const float v2 = wiener_term(*A.otf, b, xh, yh, fshift_neg(k), -kx, -ky, A.use_att != 0);
       acc = __fadd_rn(__fadd_rn(acc, v1), v2);
     }
-  const float den = __fdiv_rn(1.f, __fadd_rn(acc, wp));
+  const float den = __fdiv_rn(1.f, __fadd_rn(acc, A.wp));
   const int ax = abs(xh), ay = abs(yh);
-  const float ap = __ldg(apo + (size_t)max(ax, ay) * (W / 2 + 1) + min(ax, ay));
-  wa[((size_t)(X >> 2) * W + Y) * 4 + (X & 3)] = __fmul_rn(den, ap);
+  return __fmul_rn(den, __ldg(A.apo + (size_t)max(ax, ay) * (W / 2 + 1) + min(ax, ay)));
+}
+__global__ void k_build_wa(float* __restrict__ wa, int ncols, int W, const __grid_constant__ WaArgs A) {
+  const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y;
+  if (X >= ncols) return;
+  wa[((size_t)(X >> 2) * W + Y) * 4 + (X & 3)] = wa_at(A, X, Y, W);
+}
+// alpha and gamma of pass B1 (recon_kernels.cuh) along the output's Nyquist lines: per pair, column
+// X = N over the rows of the neg component's window, then row Y = N over its columns.
+struct PairShifts {  // the pos components' shifts [a][b-1]; a neg component has the opposite one
+  double kx[FSIM_MAX_DIRS * (FSIM_MAX_BANDS - 1)], ky[FSIM_MAX_DIRS * (FSIM_MAX_BANDS - 1)];
+};
+__global__ void k_build_edge(float4* __restrict__ edge, int W, int nWin, const int* __restrict__ win, int nPair,
+                             const __grid_constant__ PairShifts sh, const __grid_constant__ WaArgs A) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y, ab = blockIdx.z, N = W / 2;
+  if (l >= nWin) return;
+  const int band = ab % nPair + 1, cn = (ab / nPair) * (2 * nPair + 1) + 2 * band - 1;
+  const int X = row ? (win[2 * cn] + l) % W : N, Y = row ? N : (win[2 * cn + 1] + l) % W;
+  const int Xm = (W - X) % W, Ym = (W - Y) % W;
+  const double kx = sh.kx[ab], ky = sh.ky[ab];
+  const FShift kf = fshift_host(kx, ky);
+  const bool att = A.use_att != 0;
+  float2 n = make_float2(0.f, 0.f), p = make_float2(0.f, 0.f);  // OTF of neg at (X, Y), of pos at the mirrored point
+  if (!otf_at_fast(*A.otf, band, freq_x(X, W), freq_y(Y, W), fshift_neg(kf), -kx, -ky, att, &n)) n = make_float2(0.f, 0.f);
+  if (!otf_at_fast(*A.otf, band, freq_x(Xm, W), freq_y(Ym, W), kf, kx, ky, att, &p)) p = make_float2(0.f, 0.f);
+  // masks are conjugate OTFs
+  const float2 u = cscale(cconjf(n), 0.5f * wa_at(A, X, Y, W)), v = cscale(p, 0.5f * wa_at(A, Xm, Ym, W));
+  const float2 s = cadd(u, v), d = csub(u, v);
+  edge[((size_t)2 * ab + row) * nWin + l] = make_float4(s.x, s.y, d.y, -d.x);
 }
 
 // ---- plan --------------------------------------------------------------------------------------
@@ -108,6 +140,8 @@ int Plan::build(cudaStream_t st) {
   OtfTable ht;
   build_otf_table(&prm, &ht);
   const double R = ht.cutoff / ht.vec_cpm;  // OTF support radius in frequency pixels
+  const int old_nwin = nwin;
+  const int old_kind = kind();
   plan_window(&prm, R, &nwin);
   // host-side tables
   std::vector<float2> coef((size_t)nA * nC * nP);
@@ -197,10 +231,13 @@ int Plan::build(cudaStream_t st) {
   const size_t wa_elems = (size_t)(N + 4) * W, apo_elems = (size_t)(N + 1) * (N + 1);
   size_t off_nyq = off_wa + al((wa_elems + apo_elems) * sizeof(float));
   size_t off_wff = off_nyq + al(nyq.size() * sizeof(float2));
-  size_t total = off_wff + al((size_t)N * N * sizeof(float));
+  size_t off_edge = off_wff + al((size_t)N * N * sizeof(float));
+  size_t total = off_edge + al((size_t)nA * nPair * 2 * nwin * sizeof(float4));
+  const void* old_dev = dev;
   if (total > dev_bytes) {
     if (dev) cudaFree(dev);
     dev = nullptr;
+    dev_bytes = 0;
     FSIM_CUDA(fsim::dev_alloc(&dev, total));
     dev_bytes = total;
   }
@@ -214,6 +251,19 @@ int Plan::build(cudaStream_t st) {
   d_damp = fade_px > 0 ? (float*)(b + off_damp) : nullptr;
   d_masks = (float*)(b + off_mask);
   d_wa = (float*)(b + off_wa);
+  // Does a pair's support reach the output's Nyquist lines under an apodization that does too? Only
+  // such plans run pass G and the extra work of pass B1 (64 x 512^2 at 0.1 um, whose supports end at
+  // 1.13 N: 1324 us without them, 1368 with).
+  bool reach = false;
+  for (int a = 0; a < nA; a++)
+    for (int c = 1; c < nC; c++) {
+      double kx, ky;
+      comp_shift(&prm, a, c, &kx, &ky);
+      reach = reach || std::max(std::fabs(kx), std::fabs(ky)) + R > N * (1 - 1e-9);
+    }
+  reach = reach && (prm.apo_bend <= 0 || R * prm.apo_cutoff > N * (1 - 1e-9));
+  d_edge = reach ? (float4*)(b + off_edge) : nullptr;
+  if (old_dev != dev || old_nwin != nwin || old_kind != kind()) layout->fetch_add(1);
   // uploads are synchronous (pageable sources on this stack frame)
   FSIM_CUDA(cudaMemcpyAsync(d_coef, coef.data(), coef.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
   FSIM_CUDA(cudaMemcpyAsync(d_ramps, ramps.data(), ramps.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
@@ -241,9 +291,13 @@ int Plan::build(cudaStream_t st) {
     int rc = apo_octant_device(d_apo, N, ht.vec_cpm, ht.cutoff * prm.apo_cutoff, prm.apo_bend, st);
     if (rc) return rc;
     const ShiftSet sh = shift_set(&prm);
-    dim3 g(div_up(N + 4, 128), W);
-    k_build_wa<<<g, 128, 0, st>>>(d_wa, N + 4, W, d_otf, sh, fshift_set(sh), prm.use_attenuation,
-                                  (float)(prm.wiener * prm.wiener), d_apo);
+    const WaArgs A{d_otf, sh, fshift_set(sh), prm.use_attenuation, (float)(prm.wiener * prm.wiener), d_apo};
+    k_build_wa<<<dim3(div_up(N + 4, 128), W), 128, 0, st>>>(d_wa, N + 4, W, A);
+    if (d_edge) {
+      PairShifts ps;
+      for (int i = 0; i < nA * nPair; i++) comp_shift(&prm, i / nPair, 2 * (i % nPair) + 2, &ps.kx[i], &ps.ky[i]);
+      k_build_edge<<<dim3(div_up(nwin, 128), 2, nA * nPair), 128, 0, st>>>(d_edge, W, nwin, d_win, nPair, ps, A);
+    }
   }
   FSIM_CHECK_LAUNCH();
   {
@@ -292,6 +346,7 @@ void Plan::fill_job(JobDesc& j, const void* raw, float* out, float* wf, float* f
   j.nWin = nwin;
   j.status = ctx().status;
   j.cmask = otf_measured(&prm) ? 1 : 0;
+  j.edge = d_edge;
   j.clip = clip_scale;
   j.bgr = (float)bgr;
   j.damp = d_damp;
@@ -355,11 +410,11 @@ bool offline_size_supported(int n) {
 }
 
 int launch_offline_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip,
-                        int masks, bool alone, cudaStream_t st) {
+                        int kinds, bool alone, cudaStream_t st) {
   switch (n) {
 #define CASE(v) \
   case v:       \
-    return launch_offline<v>(d_jobs, njobs, maxA, maxPair, maxWin, scale_clip, masks, alone, st);
+    return launch_offline<v>(d_jobs, njobs, maxA, maxPair, maxWin, scale_clip, kinds, alone, st);
     FSIM_RECON_SIZES(CASE)
 #undef CASE
   }

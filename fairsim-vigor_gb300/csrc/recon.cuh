@@ -1,6 +1,9 @@
 // Internal interface of the fused reconstruction (recon.cu, live.cu, plan.cu).
 #pragma once
 
+#include <atomic>
+#include <memory>
+
 #include "common.cuh"
 #include "otf.cuh"
 
@@ -25,6 +28,8 @@ struct JobDesc {
   const float* wa;      // Wiener x apodization, quad layout [X/4][Y][X%4]
   const float2* nyq;    // offline: [a][b-1][x over the neg window's columns, y over its rows][nWin]: response of
                         // the neg component's odd-sample shift to the Nyquist bin (pass A)
+  const float4* edge;   // offline: [a][b-1][column X = N over the window's rows, row Y = N over its columns][nWin]:
+                        // weights of the output's Nyquist lines (pass B1); null where no support reaches them
   float2* I;            // workspace: row-transformed windows [band 0, neg of (a, b)][nWin/4][N][4] (offline);
                         // live: [band 0, pos of (a, b)][nWin/4][N][4] row, then column transforms
   float2* D;            // workspace: [a][b-1][N] Nyquist bin of every row's neg component (pass A)
@@ -41,6 +46,10 @@ struct JobDesc {
   float2* Wf;              // workspace (reused after pass C): N*N band-0 rows, then 2 x [W][N] columns
   int* status;             // the context's device status word (bounded waits that expired)
 };
+
+// Kinds of offline jobs: real or complex masks (measured OTFs), without or with edge weights. The column
+// passes have a form for each; all but the first need pass G.
+enum JobKind { JOB_REAL = 1, JOB_COMPLEX = 2, JOB_REAL_EDGE = 4, JOB_COMPLEX_EDGE = 8 };
 
 struct Plan {
   fsim_sim_param prm{};
@@ -62,6 +71,9 @@ struct Plan {
   float* d_wa = nullptr;
   float2* d_nyq = nullptr;
   float* d_wff = nullptr;  // filtered-widefield filter, N*N
+  float4* d_edge = nullptr;  // weights of the output's Nyquist lines, null where no support reaches them
+  // counts the changes of what a recorded batch holds of the plan: table addresses, window, kind
+  std::shared_ptr<std::atomic<unsigned>> layout = std::make_shared<std::atomic<unsigned>>(0);
   // host-call convenience buffers (fsim_recon_host)
   void* h_ws = nullptr;
   size_t h_ws_bytes = 0;
@@ -70,6 +82,10 @@ struct Plan {
   JobDesc* h_job = nullptr;
   JobDesc* d_job = nullptr;
 
+  int kind() const {
+    const bool c = otf_measured(&prm);
+    return d_edge ? (c ? JOB_COMPLEX_EDGE : JOB_REAL_EDGE) : (c ? JOB_COMPLEX : JOB_REAL);
+  }
   int build(cudaStream_t st);       // offline tables
   int build_live(cudaStream_t st);  // live tables
   size_t workspace_bytes() const;
@@ -91,10 +107,10 @@ bool live_size_supported(int n);
 // maxA, maxPair, maxWin: the largest angle count, band-pair count and OTF-support window
 // of the batch's datasets of size n (they bound the grids; extra blocks exit at once)
 // scale_clip: some job of the class asks for CLIPSCALE.BOTH (one more pass scales its image)
-// masks: bit 0 some job of the class has real OTF masks, bit 1 some has complex ones
+// kinds: the JobKinds of the class's jobs
 // alone: no other size class of the batch runs beside this one
 int launch_offline_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip,
-                        int masks, bool alone, cudaStream_t st);
+                        int kinds, bool alone, cudaStream_t st);
 int launch_live_size(int n, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st);
 // widefield and filtered widefield of the offline jobs that ask for them (widefield.cu);
 // launched after launch_offline_size on the same stream (it reuses the job workspaces)

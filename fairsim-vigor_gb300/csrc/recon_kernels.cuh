@@ -289,10 +289,11 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   }
 }
 
-// ---- pass G: the Nyquist column of the row transforms (complex masks only) --------------------
+// ---- pass G: the Nyquist column of the row transforms (complex masks, edge weights) ---------------------
 // A complex mask m (measured OTFs) weighs V_neg with m and V+ with conj(m), so a pair enters the
 // image as Re(m) (V_neg + V+)/2 + i Im(m) (V_neg - V+)/2 and its mirror image, and
 //   i (V_neg - V+) / 2 = Ty Qx z + Qy Tx z   (pass A's notation).
+// The same term enters the output's Nyquist column and row (pass B1) where a support reaches them.
 // Qx z is D(y) times a plan table along x: this pass transforms D along y once per angle and pair.
 template <int N, int ENV>
 __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __restrict__ jobs) {
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __rest
   load_job(&J, jobs + blockIdx.y, t, T);
   __syncthreads();
   const int nC = J.nC, nPair = (nC - 1) / 2;
-  if (!J.cmask || ab >= J.nA * nPair) return;  // uniform per block
+  if (!(J.cmask || J.edge) || ab >= J.nA * nPair) return;  // uniform per block
   const int a = ab / nPair, cn = 2 * (ab % nPair) + 1;
   const float2* d = J.D + (size_t)ab * N;
 #pragma unroll
@@ -352,9 +353,19 @@ __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __rest
 // The result over the component's row window, times its OTF mask, is the component's
 // contribution P to the image's spectrum S, stored column by column ([column][row]):
 //   H(X, Y) = S(X, Y) + conj S(-X, -Y),  S = sum of P over band 0 (mask/2) and the pairs,
-// because mask_pos(X, Y) = mask_neg(-X, -Y). With the masks and the Nyquist terms applied here,
-// where the column is in registers, pass B2 only adds windows (it took 0.358 ms per 64 datasets
-// of 512^2 3x3 while it read neg and pos masks and formed the Nyquist terms per pixel).
+// because mask_pos(X, Y) = mask_neg(-X, -Y). That fails on the output's Nyquist column X = N and row
+// Y = N: they are their own mirror images, but masks and Wiener x apodization (wa) are evaluated at
+// one coordinate of the two (-N along x, +N along y). With M = (-X, -Y), a pair's share of the image is
+//   2 H(X, Y) = f(X, Y) + conj f(M),  f(X, Y) = wa(X, Y) (m_neg(X, Y) V_neg(X, Y) + m_pos(X, Y) conj V+(M)),
+// and with V_neg = P - i G, V+ = P + i G, where P = (V_neg + V+)/2 and G is pass G's term,
+//   H(X, Y) = S(X, Y) + conj S(M),  S = alpha P + gamma G,
+//   alpha = (wa m_neg + wa(M) conj m_pos(M)) / 2,  gamma = -i (wa m_neg - wa(M) conj m_pos(M)) / 2.
+// A plan whose supports and apodization reach these lines holds alpha and gamma along them (edge): its
+// jobs run pass G, this pass weights the two lines with them and pass B2 leaves wa out there. (Band 0's
+// paste is 0 on both lines.)
+// With the masks and the Nyquist terms applied here, where the column is in registers, pass B2 only
+// adds windows (it took 0.358 ms per 64 datasets of 512^2 3x3 while it read neg and pos masks and
+// formed the Nyquist terms per pixel).
 // Adjacent columns form a line pair: CB/2 pairs of T threads per block. Each thread keeps the
 // column and then E in registers, as pass A does (in shared memory 395 us per 64 x 512^2 in place
 // of 367); the transforms' operands beside them fit 80 registers without spills worth their time
@@ -385,6 +396,36 @@ __device__ __forceinline__ void b1_put(const JobDesc& J, size_t col, int nWin, i
     out[0] = r0;
     out[nWin] = r1;
   }
+}
+// The output's Nyquist row and column among window columns xl and xl + 1 of pair ab, each weighted at its
+// own coordinates in place of the masks: rewrites what this thread has stored there. x, z: O and E of
+// this thread's rows; nyquist(yl, h): the term G.
+template <int N, int T, int EN, class F>
+__device__ __forceinline__ void b1_edges(const JobDesc& J, int ab, int xl, int t, const cpair (&x)[EN], const cpair (&z)[EN],
+                                         F nyquist) {
+  constexpr int W = 2 * N;
+  const int nWin = J.nWin, nPair = (J.nC - 1) / 2, c = (ab / nPair) * J.nC + 2 * (ab % nPair) + 1;
+  const int Xs = J.win[2 * c], Ys = J.win[2 * c + 1];
+  const int xN = Xs <= N ? N - Xs : N - Xs + W, yN = Ys <= N ? N - Ys : N - Ys + W;  // beyond nWin: not in the window
+  const float4* e = J.edge + (size_t)2 * ab * nWin;
+  float2* out = J.Tw + ((size_t)(1 + ab) * nWin + xl) * nWin;
+  auto put = [&](int yl, int h, cpair v, float4 w) {
+    float2 r[2];
+    cp_split(v, r[0], r[1]);
+    out[(size_t)h * nWin + yl] =
+        cadd(cmul(h ? r[1] : r[0], make_float2(w.x, w.y)), cmul(nyquist(yl, h), make_float2(w.z, w.w)));
+  };
+  if (t == 0 && yN < nWin)  // row N is element 0's: E - O
+    for (int h = 0; h < 2; h++) put(yN, h, csub(z[0], x[0]), __ldg(e + nWin + xl + h));
+  if ((xN & ~1) != xl || xN >= nWin) return;
+  const float2* twW = g_tw + tw_offset(W);
+#pragma unroll
+  for (int i = 0; i < EN; i++)
+    for (int yl = t + i * T - Ys + (t + i * T < Ys ? W : 0), k = 0; k < 2; k++, yl += yl < N ? N : -N) {
+      if (yl >= nWin) continue;
+      const int Y = Ys + yl < W ? Ys + yl : Ys + yl - W;
+      put(yl, xN & 1, cadd(z[i], cmul(x[i], w_dup(__ldg(twW + Y)))), __ldg(e + yl));
+    }
 }
 // elements t + i*T of window columns xl and xl + 1 from pass A's slot
 template <int N, int T, int EN>
@@ -433,7 +474,9 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
     if (paste_src<N>(Y) < 0) J.Tw[col + yl] = J.Tw[col + nWin + yl] = make_float2(0.f, 0.f);
   }
 }
-template <int N, int ENV, int CBV, bool CM>
+// EDGE: the jobs whose plans hold edge weights (a launch of their own keeps the other jobs' code as small
+// as it was: with the test in it 4 x 128^2 took 32.8 us in place of 30.8)
+template <int N, int ENV, int CBV, bool CM, bool EDGE>
 __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
     k_pass_b1(const JobDesc* __restrict__ jobs) {
   using P = Cfg<N, ENV, CBV>;
@@ -455,7 +498,7 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   // No block of this pass is launched before every block of k_pass_b0 has returned from its wait,
   // so pass A is complete by now, as the job table is; k_pass_b0's own work is not read here and is
   // only waited for before the block ends (one 256^2 stack: 34 us, 45 with the wait up here).
-  if ((J.cmask != 0) != CM /* the other launch's job */ || comp > J.nA * nPair || (int)blockIdx.x * CB >= nWin) {
+  if ((J.cmask != 0) != CM || (J.edge != nullptr) != EDGE /* another launch's job */ || comp > J.nA * nPair || (int)blockIdx.x * CB >= nWin) {
     pdl_wait();
     return;  // uniform per block
   }
@@ -492,12 +535,12 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
   }
   line_fft_pair<N, T, CP, false>(x, s, lane, t, twN);  // Z along y
   const float2* nx = J.nyq + (size_t)ab * 2 * nWin;  // Qx over the window columns, Qy over its rows
-  __shared__ float2 szc[CM ? CB : 1];
+  __shared__ float2 szc[CM || EDGE ? CB : 1];
   cpair zq = cp_zero();
   if (t == (N / 2) % T) {
     float2 z = part[0];
     for (int k = 1; k < (NT + 31) / 32; k++) z = cadd(z, part[k]);
-    if constexpr (CM) cp_split(x[(N / 2) / T], szc[2 * lane], szc[2 * lane + 1]);  // read after barriers
+    if constexpr (CM || EDGE) cp_split(x[(N / 2) / T], szc[2 * lane], szc[2 * lane + 1]);  // read after barriers
     z = make_float2(-z.x, -z.y);
     zq = cp_make(cmul(z, __ldg(nx + xl)), cmul(z, __ldg(nx + xl + 1)));
   }
@@ -539,6 +582,11 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
       if (yl + N < nWin) finish(yl + N, csub(z[i], o));
     }
   }
+  if constexpr (EDGE) {
+    b1_edges<N, T>(J, ab, xl, t, x, z, [&](int yl, int h) {
+      return cadd(cmul(__ldg(nx + xl + h), J.G[(size_t)ab * nWin + yl]), cmul(__ldg(nx + nWin + yl), szc[2 * lane + h]));
+    });
+  }
   pdl_wait();
 }
 
@@ -562,7 +610,7 @@ struct PassB2 {
   // one block per SM, and 64 leave two (a 2048^2 3x5 stack: 94 -> 86 us)
   static constexpr int MINB = pair_min_blocks(NT, P::EN, NT >= 512 ? 64 : 80);
 };
-template <int N, int ENV, int CBV>
+template <int N, int ENV, int CBV, bool EDGE>
 __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::MINB)
     k_pass_b2(const JobDesc* __restrict__ jobs) {
   using P = Cfg<N, ENV, CBV>;
@@ -577,6 +625,7 @@ __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::
   pdl_trigger();
   pdl_wait();
   __syncthreads();
+  if ((J.edge != nullptr) != EDGE) return;  // another launch's job (uniform per block)
   const int nC = J.nC, nWin = J.nWin, nPair = (nC - 1) / 2, nS = 1 + J.nA * nPair;
   auto wrap = [](int v) { return v < 0 ? v + W : (v >= W ? v - W : v); };
   const int Xm = wrap(-X);
@@ -624,7 +673,11 @@ __global__ void __launch_bounds__(PassB2<N, ENV, CBV>::NT, PassB2<N, ENV, CBV>::
 #pragma unroll
   for (int i = 0; i < EN; i++) {
     const int k = t + i * T;
-    const float f0 = __ldg(wa + (size_t)k * 4), f1 = __ldg(wa + (size_t)(k + N) * 4);
+    float f0 = __ldg(wa + (size_t)k * 4), f1 = __ldg(wa + (size_t)(k + N) * 4);
+    if constexpr (EDGE) {  // pass B1 has weighted the Nyquist column and row
+      if (X == N) f0 = f1 = 1.f;
+      if (k == 0) f1 = 1.f;
+    }
     const float2 u0 = cscale(acc[0][i], f0), u1 = cscale(acc[1][i], f1);
     x[i] = cp_make(cadd(u0, u1), cmul(csub(u0, u1), cconjf(__ldg(twW + k))));
   }
@@ -713,7 +766,7 @@ static __global__ void k_scale_clip(const JobDesc* __restrict__ jobs, int W) {
 
 // ---- launch ----------------------------------------------------------------------------------------
 // Each pass has its own launch-shape variants (autotuner: tuning.json); a batch launches
-// A, (G,) B1, B2, C in order on one stream; G only where some job has complex masks.
+// A, (G,) B1, B2, C in order on one stream; G only where some job needs it.
 // Dynamic shared memory of a kernel instantiation, granted once per process.
 template <class K>
 static int grant_smem(K kern, size_t bytes, bool& done) {
@@ -740,35 +793,47 @@ static void launch_g(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, cu
   k_pass_g<N, ENA><<<dim3(maxA * maxPair, njobs), PA::T, 0, st>>>(d_jobs);
 }
 template <int N, int ENB, int CBB, bool CM>
-static int launch_b1_kind(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
+static int launch_b0(bool dep, const JobDesc* d_jobs, int njobs, int maxWin, cudaStream_t st) {
   using PB = PassB1<N, ENB, CBB>;
   constexpr int CB = 2 * PB::CP;
-  static bool attr = false, attr0 = false;
-  int rc = grant_smem(k_pass_b1<N, ENB, CBB, CM>, PB::SMEM, attr);
-  if (!rc) rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM, attr0);
+  static bool attr = false;
+  int rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM, attr);
   if (rc) return rc;
   FSIM_CUDA(launch_pass(dep, k_pass_b0<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM, st,
                         d_jobs));
-  FSIM_CUDA(launch_pass(dep, k_pass_b1<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT,
+  return FSIM_OK;
+}
+template <int N, int ENB, int CBB, bool CM, bool EDGE>
+static int launch_b1_pairs(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
+  using PB = PassB1<N, ENB, CBB>;
+  constexpr int CB = 2 * PB::CP;
+  static bool attr = false;
+  int rc = grant_smem(k_pass_b1<N, ENB, CBB, CM, EDGE>, PB::SMEM, attr);
+  if (rc) return rc;
+  FSIM_CUDA(launch_pass(dep, k_pass_b1<N, ENB, CBB, CM, EDGE>, dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT,
                         PB::SMEM, st, d_jobs));
   return FSIM_OK;
 }
-// masks: bit 0 launches the real-mask kind, bit 1 the complex-mask kind (measured OTFs)
-template <int N, int ENB, int CBB>
-static int launch_b1(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int masks, cudaStream_t st) {
+// kinds: JOB_REAL | JOB_COMPLEX, or with EDGE the other two
+template <int N, int ENB, int CBB, bool EDGE>
+static int launch_b1(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int kinds, cudaStream_t st) {
   int rc = FSIM_OK;
-  if (masks & 1) rc = launch_b1_kind<N, ENB, CBB, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
-  if (!rc && (masks & 2)) rc = launch_b1_kind<N, ENB, CBB, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!EDGE && (kinds & (JOB_REAL | JOB_REAL_EDGE))) rc = launch_b0<N, ENB, CBB, false>(dep, d_jobs, njobs, maxWin, st);
+  if (!rc && (kinds & (EDGE ? JOB_REAL_EDGE : JOB_REAL)))
+    rc = launch_b1_pairs<N, ENB, CBB, false, EDGE>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && !EDGE && (kinds & (JOB_COMPLEX | JOB_COMPLEX_EDGE))) rc = launch_b0<N, ENB, CBB, true>(dep, d_jobs, njobs, maxWin, st);
+  if (!rc && (kinds & (EDGE ? JOB_COMPLEX_EDGE : JOB_COMPLEX)))
+    rc = launch_b1_pairs<N, ENB, CBB, true, EDGE>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
   return rc;
 }
-template <int N, int ENB, int CBB>
+template <int N, int ENB, int CBB, bool EDGE>
 static int launch_b2(bool dep, const JobDesc* d_jobs, int njobs, cudaStream_t st) {
   using PB = PassB2<N, ENB, CBB>;
   constexpr int CB = Cfg<N, ENB, CBB>::CB;
   static bool attr = false;
-  int rc = grant_smem(k_pass_b2<N, ENB, CBB>, PB::SMEM, attr);
+  int rc = grant_smem(k_pass_b2<N, ENB, CBB, EDGE>, PB::SMEM, attr);
   if (rc) return rc;
-  FSIM_CUDA(launch_pass(dep, k_pass_b2<N, ENB, CBB>, dim3(N / CB + 1, njobs), PB::NT, PB::SMEM, st, d_jobs));  // 0..N
+  FSIM_CUDA(launch_pass(dep, k_pass_b2<N, ENB, CBB, EDGE>, dim3(N / CB + 1, njobs), PB::NT, PB::SMEM, st, d_jobs));  // 0..N
   return FSIM_OK;
 }
 
@@ -793,7 +858,7 @@ __host__ inline int size_slot(int n) {
 // (elements, columns per block) {(E0,4), (E0,2), (E1,4), (E1,2)} with E0 = 8, E1 = 16
 // (3*2^k sizes: 12, 24). The extremes (N <= 128, N >= 2048) have one variant.
 template <int N>
-int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip, int masks,
+int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip, int kinds,
                    bool alone, cudaStream_t st) {
   constexpr bool p3 = (N % 3 == 0);
   constexpr int E0 = p3 ? 12 : 8, E1 = p3 ? 24 : 16;
@@ -812,32 +877,37 @@ int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int 
   else if constexpr (!single) rc = launch_a<N, E1>(d_jobs, njobs, maxA, st);
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[1], st);
-  if (masks & 2) {
+  if (kinds & ~JOB_REAL) {
     if (va == 0) launch_g<N, E0>(d_jobs, njobs, maxA, maxPair, st);
     else if constexpr (!single) launch_g<N, E1>(d_jobs, njobs, maxA, maxPair, st);
   }
+  const bool edge = kinds & (JOB_REAL_EDGE | JOB_COMPLEX_EDGE), plain = kinds & (JOB_REAL | JOB_COMPLEX);
   if constexpr (single) {
-    rc = launch_b1<N, E0, CBX>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st);
+    rc = launch_b1<N, E0, CBX, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st);
   } else {
     switch (vb1) {
-      case 0: rc = launch_b1<N, E0, 4>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      case 1: rc = launch_b1<N, E0, 2>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      case 2: rc = launch_b1<N, E1, 4>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
-      default: rc = launch_b1<N, E1, 2>(dep, d_jobs, njobs, maxA, maxPair, maxWin, masks, st); break;
+      case 0: rc = launch_b1<N, E0, 4, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+      case 1: rc = launch_b1<N, E0, 2, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+      case 2: rc = launch_b1<N, E1, 4, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+      default: rc = launch_b1<N, E1, 2, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
     }
   }
+  if (!rc && edge) rc = launch_b1<N, E0, CBX, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st);  // one variant
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[2], st);
-  if constexpr (single) {
-    rc = launch_b2<N, E0, CBX>(dep, d_jobs, njobs, st);
-  } else {
-    switch (vb2) {
-      case 0: rc = launch_b2<N, E0, 4>(dep, d_jobs, njobs, st); break;
-      case 1: rc = launch_b2<N, E0, 2>(dep, d_jobs, njobs, st); break;
-      case 2: rc = launch_b2<N, E1, 4>(dep, d_jobs, njobs, st); break;
-      default: rc = launch_b2<N, E1, 2>(dep, d_jobs, njobs, st); break;
+  if (plain) {
+    if constexpr (single) {
+      rc = launch_b2<N, E0, CBX, false>(dep, d_jobs, njobs, st);
+    } else {
+      switch (vb2) {
+        case 0: rc = launch_b2<N, E0, 4, false>(dep, d_jobs, njobs, st); break;
+        case 1: rc = launch_b2<N, E0, 2, false>(dep, d_jobs, njobs, st); break;
+        case 2: rc = launch_b2<N, E1, 4, false>(dep, d_jobs, njobs, st); break;
+        default: rc = launch_b2<N, E1, 2, false>(dep, d_jobs, njobs, st); break;
+      }
     }
   }
+  if (!rc && edge) rc = launch_b2<N, E0, CBX, true>(dep, d_jobs, njobs, st);
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[3], st);
   using PC = Cfg<N>;
