@@ -142,7 +142,6 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
   ulonglong2* s = smp + g * PA::XS;
   const float2* twN = g_stw + stw_offset(N, EN);  // stage table, read through L1
   const float2* twW = g_tw + tw_offset(W);
-  pdl_trigger();
   const JobDesc* jg = jobs + blockIdx.z;
   load_job(&J, jg, tid, NT);
   // the counts and the separation coefficients straight from the descriptor in global
@@ -287,6 +286,9 @@ __global__ void __launch_bounds__(PassA<N, ENV>::NT, PassA<N, ENV>::MINB) k_pass
       }
     }
   }
+  // At its end, as pass B's: blocks that start early are placed on SMs that still run this pass and
+  // wait there (4 x 128^2 30.7 us, 39.5 with this at the start; one 192^2 stack 41.0, 47.4).
+  pdl_trigger();
 }
 
 // ---- pass G: the Nyquist column of the row transforms (complex masks, edge weights) ---------------------
@@ -305,6 +307,8 @@ __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __rest
   const float2* twN = g_stw + stw_offset(N, EN);
   const float2* twW = g_tw + tw_offset(W);
   load_job(&J, jobs + blockIdx.y, t, T);
+  pdl_trigger();
+  pdl_wait();
   __syncthreads();
   const int nC = J.nC, nPair = (nC - 1) / 2;
   if (!(J.cmask || J.edge) || ab >= J.nA * nPair) return;  // uniform per block
@@ -347,9 +351,9 @@ __global__ void __launch_bounds__(Cfg<N, ENV>::T) k_pass_g(const JobDesc* __rest
 }
 
 // ---- pass B1: column transforms of band 0 and of the neg components, masked ---------------------
-// One block per CB window columns of one component: band 0 (k_pass_b0; the windows of all angles
-// summed: they share one unshifted mask) is transformed along y and pasted; each pair's neg
-// component (k_pass_b1) gets the full y shift (even/odd split, the Nyquist bin as pass A's comment says).
+// One block per CB window columns of one component: band 0 (the windows of all angles summed: they
+// share one unshifted mask) is transformed along y and pasted; each pair's neg component gets the
+// full y shift (even/odd split, the Nyquist bin as pass A's comment says).
 // The result over the component's row window, times its OTF mask, is the component's
 // contribution P to the image's spectrum S, stored column by column ([column][row]):
 //   H(X, Y) = S(X, Y) + conj S(-X, -Y),  S = sum of P over band 0 (mask/2) and the pairs,
@@ -440,26 +444,14 @@ __device__ __forceinline__ void b1_load(const JobDesc& J, int slot, int nWin, in
 }
 // Band 0: summed over the angles and row-transformed in pass A (slot 0); one transform per column.
 template <int N, int ENV, int CBV, bool CM>
-__global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
-    k_pass_b0(const JobDesc* __restrict__ jobs) {
+__device__ __forceinline__ void b1_band0(const JobDesc& J, int xl, int lane, int t, ulonglong2* s) {
   using P = Cfg<N, ENV, CBV>;
-  using PB = PassB1<N, ENV, CBV>;
-  constexpr int W = P::W, T = P::T, CB = P::CB, EN = P::EN, CP = PB::CP, NT = PB::NT;
-  const int lt = threadIdx.x, lane = lt % CP, t = lt / CP;
-  __shared__ JobDesc J;
-  extern __shared__ ulonglong2 smp[];
-  load_job(&J, jobs + blockIdx.y, lt, NT);  // written before pass A
-  __syncthreads();
-  pdl_wait();
-  pdl_trigger();  // pass B1 may start: pass A is complete
-  if ((J.cmask != 0) != CM) return;  // the other launch's job (uniform per block)
+  constexpr int W = P::W, T = P::T, EN = P::EN, CP = PassB1<N, ENV, CBV>::CP;
   const int nWin = J.nWin;
-  if ((int)blockIdx.x * CB >= nWin) return;  // uniform per block
-  const int xl = blockIdx.x * CB + 2 * lane;  // and xl + 1; nWin is a multiple of 4: both are inside
   const size_t col = (size_t)xl * nWin;
   cpair x[EN];
   b1_load<N, T, EN>(J, 0, nWin, xl, t, x);
-  line_fft_pair<N, T, CP, false>(x, smp, lane, t, g_stw + stw_offset(N, EN));
+  line_fft_pair<N, T, CP, false>(x, s, lane, t, g_stw + stw_offset(N, EN));
   const int Ys = J.win[1];
 #pragma unroll
   for (int i = 0; i < EN; i++) {
@@ -474,35 +466,21 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
     if (paste_src<N>(Y) < 0) J.Tw[col + yl] = J.Tw[col + nWin + yl] = make_float2(0.f, 0.f);
   }
 }
-// EDGE: the jobs whose plans hold edge weights (a launch of their own keeps the other jobs' code as small
-// as it was: with the test in it 4 x 128^2 took 32.8 us in place of 30.8)
+template <int N, int ENV, int CBV, bool CM>
+__device__ __noinline__ void b1_band0_call(const JobDesc& J, int xl, int lane, int t, ulonglong2* s) {
+  b1_band0<N, ENV, CBV, CM>(J, xl, lane, t, s);
+}
+// The neg component comp = 1 + a*nPair + (b-1) of (a, b), window columns xl and xl + 1.
 template <int N, int ENV, int CBV, bool CM, bool EDGE>
-__global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
-    k_pass_b1(const JobDesc* __restrict__ jobs) {
+__device__ __forceinline__ void b1_pair(const JobDesc& J, int comp, int xl, int lt, ulonglong2* s) {
   using P = Cfg<N, ENV, CBV>;
   using PB = PassB1<N, ENV, CBV>;
   constexpr int W = P::W, T = P::T, CB = P::CB, EN = P::EN, CP = PB::CP, NT = PB::NT, WS = NT < 32 ? NT : 32;
-  const int lt = threadIdx.x, lane = lt % CP, t = lt / CP;
-  __shared__ JobDesc J;
+  const int lane = lt % CP, t = lt / CP, nC = J.nC, nWin = J.nWin, nPair = (nC - 1) / 2;
   __shared__ float2 part[(NT + 31) / 32];
-  extern __shared__ ulonglong2 smp[];
-  ulonglong2* s = smp;
   cpair z[EN];
   const float2* twN = g_stw + stw_offset(N, EN);
   const float2* twW = g_tw + tw_offset(W);
-  load_job(&J, jobs + blockIdx.z, lt, NT);
-  pdl_trigger();
-  __syncthreads();
-  const int nC = J.nC, nWin = J.nWin, nPair = (nC - 1) / 2;
-  const int comp = 1 + blockIdx.y;  // 1 + a*nPair + (b-1): neg of (a, b)
-  // No block of this pass is launched before every block of k_pass_b0 has returned from its wait,
-  // so pass A is complete by now, as the job table is; k_pass_b0's own work is not read here and is
-  // only waited for before the block ends (one 256^2 stack: 34 us, 45 with the wait up here).
-  if ((J.cmask != 0) != CM || (J.edge != nullptr) != EDGE /* another launch's job */ || comp > J.nA * nPair || (int)blockIdx.x * CB >= nWin) {
-    pdl_wait();
-    return;  // uniform per block
-  }
-  const int xl = blockIdx.x * CB + 2 * lane;  // and xl + 1; nWin is a multiple of 4: both are inside
   const size_t col = ((size_t)comp * nWin + xl) * nWin;
   cpair x[EN];  // element t + i*T of this lane's columns, in registers through the transforms
   b1_load<N, T, EN>(J, comp, nWin, xl, t, x);
@@ -587,7 +565,59 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
       return cadd(cmul(__ldg(nx + xl + h), J.G[(size_t)ab * nWin + yl]), cmul(__ldg(nx + nWin + yl), szc[2 * lane + h]));
     });
   }
+}
+
+template <int N, int ENV, int CBV, bool CM>
+__global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
+    k_pass_b0(const JobDesc* __restrict__ jobs) {
+  using P = Cfg<N, ENV, CBV>;
+  using PB = PassB1<N, ENV, CBV>;
+  const int lt = threadIdx.x, x0 = blockIdx.x * P::CB;
+  __shared__ JobDesc J;
+  extern __shared__ ulonglong2 smp[];
+  load_job(&J, jobs + blockIdx.y, lt, PB::NT);
+  __syncthreads();
+  if ((J.cmask != 0) != CM || J.edge || x0 >= J.nWin) return;  // another launch's job (uniform per block)
+  // the thread's columns xl and xl + 1: nWin is a multiple of 4, both are inside
+  b1_band0<N, ENV, CBV, CM>(J, x0 + 2 * (lt % PB::CP), lt % PB::CP, lt / PB::CP, smp);
+}
+template <int N, int ENV, int CBV, bool CM>
+__global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
+    k_pass_b1(const JobDesc* __restrict__ jobs) {
+  using P = Cfg<N, ENV, CBV>;
+  using PB = PassB1<N, ENV, CBV>;
+  const int lt = threadIdx.x, x0 = blockIdx.x * P::CB, comp = 1 + blockIdx.y;
+  __shared__ JobDesc J;
+  extern __shared__ ulonglong2 smp[];
+  load_job(&J, jobs + blockIdx.z, lt, PB::NT);
+  __syncthreads();
+  if ((J.cmask != 0) != CM || J.edge || comp > J.nA * (J.nC - 1) / 2 || x0 >= J.nWin) return;  // uniform per block
+  b1_pair<N, ENV, CBV, CM, false>(J, comp, x0 + 2 * (lt % PB::CP), lt, smp);
+}
+// Band 0 and the pairs in one launch: the form of dependent launches, whose blocks all wait for pass A
+// (and G) before they read what it wrote, and of the jobs with edge weights (EDGE). Band 0, the shorter
+// work, comes last: of each job at 3*2^k lengths, of all jobs at 2^k (4 x 1024^2 359 us, 364 job by job, but 4 x
+// 768^2 230 job by job and 242 the other way). In long batches the two kernels are faster: band 0 by itself
+// needs fewer registers (16 x 512^2 306 us, 309 in one).
+template <int N, int ENV, int CBV, bool CM, bool EDGE>
+__global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
+    k_pass_b01(const JobDesc* __restrict__ jobs) {
+  using P = Cfg<N, ENV, CBV>;
+  using PB = PassB1<N, ENV, CBV>;
+  constexpr bool BYJOB = N % 3 == 0;
+  const int lt = threadIdx.x, x0 = blockIdx.x * P::CB;
+  const int c = BYJOB ? blockIdx.y : blockIdx.z, comp = c + 1 < (int)(BYJOB ? gridDim.y : gridDim.z) ? c + 1 : 0;
+  __shared__ JobDesc J;
+  extern __shared__ ulonglong2 smp[];
+  load_job(&J, jobs + (BYJOB ? blockIdx.z : blockIdx.y), lt, PB::NT);  // written before pass A
   pdl_wait();
+  __syncthreads();
+  if ((J.cmask != 0) != CM || (J.edge != nullptr) != EDGE || comp > J.nA * (J.nC - 1) / 2 || x0 >= J.nWin)
+    return;  // uniform per block
+  const int lane = lt % PB::CP, xl = x0 + 2 * lane;
+  if (comp == 0) b1_band0_call<N, ENV, CBV, CM>(J, xl, lane, lt / PB::CP, smp);
+  else b1_pair<N, ENV, CBV, CM, EDGE>(J, comp, xl, lt, smp);
+  pdl_trigger();
 }
 
 // ---- pass B2: Hermitian sum over components, Wiener x apodization, inverse along y -------------
@@ -788,42 +818,52 @@ static int launch_a(const JobDesc* d_jobs, int njobs, int maxA, cudaStream_t st)
 }
 
 template <int N, int ENA>
-static void launch_g(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, cudaStream_t st) {
-  using PA = Cfg<N, ENA>;
-  k_pass_g<N, ENA><<<dim3(maxA * maxPair, njobs), PA::T, 0, st>>>(d_jobs);
+static int launch_g(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, cudaStream_t st) {
+  FSIM_CUDA(launch_pass(dep, k_pass_g<N, ENA>, dim3(maxA * maxPair, njobs), Cfg<N, ENA>::T, 0, st, d_jobs));
+  return FSIM_OK;
 }
+// Band 0 and the pairs of one kind of jobs: two launches, or one (k_pass_b01).
 template <int N, int ENB, int CBB, bool CM>
-static int launch_b0(bool dep, const JobDesc* d_jobs, int njobs, int maxWin, cudaStream_t st) {
+static int launch_b_two(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
   using PB = PassB1<N, ENB, CBB>;
   constexpr int CB = 2 * PB::CP;
-  static bool attr = false;
-  int rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM, attr);
+  static bool attr0 = false, attr = false;
+  int rc = grant_smem(k_pass_b0<N, ENB, CBB, CM>, PB::SMEM, attr0);
+  if (!rc) rc = grant_smem(k_pass_b1<N, ENB, CBB, CM>, PB::SMEM, attr);
   if (rc) return rc;
-  FSIM_CUDA(launch_pass(dep, k_pass_b0<N, ENB, CBB, CM>, dim3((maxWin + CB - 1) / CB, njobs), PB::NT, PB::SMEM, st,
-                        d_jobs));
+  const int gx = (maxWin + CB - 1) / CB;
+  k_pass_b0<N, ENB, CBB, CM><<<dim3(gx, njobs), PB::NT, PB::SMEM, st>>>(d_jobs);
+  k_pass_b1<N, ENB, CBB, CM><<<dim3(gx, maxA * maxPair, njobs), PB::NT, PB::SMEM, st>>>(d_jobs);
   return FSIM_OK;
 }
 template <int N, int ENB, int CBB, bool CM, bool EDGE>
-static int launch_b1_pairs(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
+static int launch_b_one(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, cudaStream_t st) {
   using PB = PassB1<N, ENB, CBB>;
   constexpr int CB = 2 * PB::CP;
   static bool attr = false;
-  int rc = grant_smem(k_pass_b1<N, ENB, CBB, CM, EDGE>, PB::SMEM, attr);
+  int rc = grant_smem(k_pass_b01<N, ENB, CBB, CM, EDGE>, PB::SMEM, attr);
   if (rc) return rc;
-  FSIM_CUDA(launch_pass(dep, k_pass_b1<N, ENB, CBB, CM, EDGE>, dim3((maxWin + CB - 1) / CB, maxA * maxPair, njobs), PB::NT,
-                        PB::SMEM, st, d_jobs));
+  const int gx = (maxWin + CB - 1) / CB, comps = 1 + maxA * maxPair;
+  FSIM_CUDA(launch_pass(dep, k_pass_b01<N, ENB, CBB, CM, EDGE>, N % 3 == 0 ? dim3(gx, comps, njobs) : dim3(gx, njobs, comps),
+                        PB::NT, PB::SMEM, st, d_jobs));
   return FSIM_OK;
 }
-// kinds: JOB_REAL | JOB_COMPLEX, or with EDGE the other two
-template <int N, int ENB, int CBB, bool EDGE>
-static int launch_b1(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int kinds, cudaStream_t st) {
+// jobs without edge weights, in long batches
+template <int N, int ENB, int CBB>
+static int launch_b1(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int kinds, cudaStream_t st) {
   int rc = FSIM_OK;
-  if (!EDGE && (kinds & (JOB_REAL | JOB_REAL_EDGE))) rc = launch_b0<N, ENB, CBB, false>(dep, d_jobs, njobs, maxWin, st);
-  if (!rc && (kinds & (EDGE ? JOB_REAL_EDGE : JOB_REAL)))
-    rc = launch_b1_pairs<N, ENB, CBB, false, EDGE>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
-  if (!rc && !EDGE && (kinds & (JOB_COMPLEX | JOB_COMPLEX_EDGE))) rc = launch_b0<N, ENB, CBB, true>(dep, d_jobs, njobs, maxWin, st);
-  if (!rc && (kinds & (EDGE ? JOB_COMPLEX_EDGE : JOB_COMPLEX)))
-    rc = launch_b1_pairs<N, ENB, CBB, true, EDGE>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (kinds & JOB_REAL) rc = launch_b_two<N, ENB, CBB, false>(d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && (kinds & JOB_COMPLEX)) rc = launch_b_two<N, ENB, CBB, true>(d_jobs, njobs, maxA, maxPair, maxWin, st);
+  return rc;
+}
+// the same in one launch, and the jobs with edge weights: one variant
+template <int N, int ENB, int CBB>
+static int launch_b01(bool dep, const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, int kinds, cudaStream_t st) {
+  int rc = FSIM_OK;
+  if (kinds & JOB_REAL) rc = launch_b_one<N, ENB, CBB, false, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && (kinds & JOB_COMPLEX)) rc = launch_b_one<N, ENB, CBB, true, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && (kinds & JOB_REAL_EDGE)) rc = launch_b_one<N, ENB, CBB, false, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
+  if (!rc && (kinds & JOB_COMPLEX_EDGE)) rc = launch_b_one<N, ENB, CBB, true, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, st);
   return rc;
 }
 template <int N, int ENB, int CBB, bool EDGE>
@@ -878,21 +918,25 @@ int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int 
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[1], st);
   if (kinds & ~JOB_REAL) {
-    if (va == 0) launch_g<N, E0>(d_jobs, njobs, maxA, maxPair, st);
-    else if constexpr (!single) launch_g<N, E1>(d_jobs, njobs, maxA, maxPair, st);
+    if (va == 0) rc = launch_g<N, E0>(dep, d_jobs, njobs, maxA, maxPair, st);
+    else if constexpr (!single) rc = launch_g<N, E1>(dep, d_jobs, njobs, maxA, maxPair, st);
+    if (rc) return rc;
   }
   const bool edge = kinds & (JOB_REAL_EDGE | JOB_COMPLEX_EDGE), plain = kinds & (JOB_REAL | JOB_COMPLEX);
-  if constexpr (single) {
-    rc = launch_b1<N, E0, CBX, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st);
-  } else {
-    switch (vb1) {
-      case 0: rc = launch_b1<N, E0, 4, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
-      case 1: rc = launch_b1<N, E0, 2, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
-      case 2: rc = launch_b1<N, E1, 4, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
-      default: rc = launch_b1<N, E1, 2, false>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+  if (!dep) {
+    if constexpr (single) {
+      rc = launch_b1<N, E0, CBX>(d_jobs, njobs, maxA, maxPair, maxWin, kinds, st);
+    } else {
+      switch (vb1) {
+        case 0: rc = launch_b1<N, E0, 4>(d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+        case 1: rc = launch_b1<N, E0, 2>(d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+        case 2: rc = launch_b1<N, E1, 4>(d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+        default: rc = launch_b1<N, E1, 2>(d_jobs, njobs, maxA, maxPair, maxWin, kinds, st); break;
+      }
     }
   }
-  if (!rc && edge) rc = launch_b1<N, E0, CBX, true>(dep, d_jobs, njobs, maxA, maxPair, maxWin, kinds, st);  // one variant
+  const int one = dep ? kinds : kinds & (JOB_REAL_EDGE | JOB_COMPLEX_EDGE);
+  if (!rc && one) rc = launch_b01<N, E0, CBX>(dep, d_jobs, njobs, maxA, maxPair, maxWin, one, st);
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[2], st);
   if (plain) {

@@ -91,3 +91,25 @@ def test_output_nyquist_after_plan_update(fs, oracle, torch_cuda):
         g.launch()
         torch.cuda.synchronize()
         assert rel_l2(d_out.cpu().numpy(), exp) < 1e-5
+
+
+@pytest.mark.parametrize("pixel,measured", [(0.08, True), (0.12, False), (0.10, True)])
+def test_short_and_long_batches_same_bits(fs, torch_cuda, pixel, measured):
+    """Short batches run band 0 and the pairs as one dependent launch behind passes A and G, long ones as
+    two launches: the same bits with complex masks and edge weights too (real masks inside the grid
+    in test_gpu_short_batches.py)."""
+    torch = torch_cuda
+    n, count = 64, 640
+    raw, sp = _make(fs, n, 21, pixel, measured=measured)
+    plan = _plan(fs, sp)
+    gain = torch.linspace(0.5, 2.0, count, device="cuda").view(-1, 1, 1, 1)
+    d_raw = (torch.from_numpy(raw).cuda().reshape(1, -1, n, n) * gain).contiguous()
+    out = torch.empty((2, count, 2 * n, 2 * n), dtype=torch.float32, device="cuda")
+    ws = torch.empty(fs.plan.batch_workspace_bytes([plan] * count), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for dst, step in zip(out, (count, 5)):
+        for k in range(0, count, step):
+            fs.plan.recon_batch([(plan, d_raw[i].data_ptr(), dst[i].data_ptr()) for i in range(k, k + step)],
+                                ws.data_ptr(), ws.numel())
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1])
