@@ -330,9 +330,9 @@ __global__ void __launch_bounds__(FCfg<N>::G* FCfg<N>::T, FCfg<N>::blocks(FCfg<N
       for (int w = P::PT; w < T; w += P::PT) f += pv[w + l + h];
       d += f;
     }
-    const unsigned act = __activemask();  // whole groups of four: T and 4 * NV are multiples of 4
-    d += __shfl_xor_sync(act, d, 1);
-    d += __shfl_xor_sync(act, d, 2);
+    const unsigned four = 0xfu << (threadIdx.x & 28);  // enter together: T and 4 * NV are multiples of 4
+    d += __shfl_xor_sync(four, d, 1);
+    d += __shfl_xor_sync(four, d, 2);
     if (h == 0) {
       if (v == 2 * NG) A.n2[(size_t)a * N + y] = d;
       else reinterpret_cast<double*>(A.Q + ((size_t)a * NG + v / 2) * N + y)[v & 1] = d;
