@@ -13,10 +13,11 @@
 //            grid point: the sum over rows, the last block to finish scans the grid in the
 //            reference's order and sets up the next step
 //   getPeak  region, two-pass inverse transforms and row sums as Correlation.getPeak's vector form
-// The search only picks grid points, so its roundings do not show in the result; the spectra and
-// getPeak, whose phase and modulation are reported in double, keep the roundings of the form that
-// ran one vector operation at a time (transforms line by line, sums in its order). That form took
-// 2.87 ms at 1024^2 (3 x 3, f32): 13 launches per search step and direction, each pass over memory.
+// The search's transforms run on pairs, so its own phase and magnitude (reported with the peaks) carry
+// other roundings of the same size as the form that ran one vector operation at a time; ramps, products
+// and sums hold what they held there. The spectra and getPeak, whose phase and modulation the fit
+// stores, keep that form's roundings (transforms line by line, sums in its order). It took 2.87 ms at
+// 1024^2 (3 x 3, f32): 13 launches per search step and direction, each pass over memory.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -37,7 +38,8 @@ namespace fsim {
 namespace {
 
 constexpr int NG = 10;       // grid side of a search step (Correlation.fitPeak)
-constexpr int NV = 2 * NG + 1;  // sums per row: NG complex ramp sums, norm2
+constexpr int NV = 2 * NG;   // sums per row: NG complex ramp sums (norm2 has its own)
+constexpr int NR = 2 * NG;   // ramps per direction: the grid's columns, then its rows
 
 // One direction's state: the search of the current step (position, width, shifts, common region)
 // and the best correlation so far.
@@ -55,7 +57,9 @@ struct FitArgs {  // what the passes need besides planes and state
   const float* weight;   // 1 / OTF inside the weight limit, 0 beyond, N*N (symmetric)
   float wlf;             // weight limit: the smallest float >= it
   float d2_keep, d2_drop;  // squared distance (px^2) surely inside / beyond the weight limit; d2_drop < 0: unknown
-  float2* ramps;         // per direction: 3 x ramps, then NG y ramps, N entries each
+  // Per direction NR ramps of N entries. Search: x ramps j and j + NG/2 together, {re, re, im, im} per
+  // entry, then the y ramps one by one. getPeak: its x ramp first, its y ramp at NG * N.
+  float2* ramps;
   double2* Q;            // per direction: NG x N row sums
   double* n2;            // per direction: N row norms
   float* pmag;           // per direction and peak block
@@ -170,42 +174,55 @@ __device__ __forceinline__ float2 ramp_at(double k, int x, int N) {  // exp(2 pi
   sincospi(2.0 * f, &s, &c);
   return make_float2((float)c, (float)s);
 }
-// The search's ramps: the phase is reduced in double, its sine and cosine taken in float at the
-// phase's float part and carried to the rest of it by the first derivative (within 2 ulp). In FP64 (two
-// operations per clock and SM on GB300) the ramps of a step took longer than its column pass.
-__device__ __forceinline__ float2 ramp_search(double k, int x, double inv_n) {
-  double f = k * ((double)x * inv_n);
-  f -= rint(f);
-  const float h = (float)f, l = (float)(f - (double)h) * 6.2831853f;
-  float s, c;
-  sincospif(2.f * h, &s, &c);
-  return make_float2(c - l * s, s + l * c);
+// One ramp of the search by a block, in FP64 and rounded once, as ramp_at: exp(2 pi i k (32 m + l) / N) is
+// the product of two factors out of N/32 + 32. (GB300 runs two FP64 operations per clock and SM: with a
+// sine and cosine for every entry the ramps of a step took longer than its column pass.)
+__device__ __forceinline__ double2 turn(double f) {
+  f -= floor(f);
+  double s, c;
+  sincospi(2.0 * f, &s, &c);
+  return make_double2(c, s);
 }
-// SEARCH false: times the attenuation, inverse. true: common region, inverse; the first RB blocks of a
+template <class F>
+__device__ __forceinline__ void ramp_search(double k, int N, double2* f, F put) {
+  const int nh = N / 32;
+  for (int i = threadIdx.x; i < nh + 32; i += blockDim.x) f[i] = turn(k * (double)(i < nh ? 32 * i : i - nh) / (double)N);
+  __syncthreads();
+  for (int x = threadIdx.x; x < N; x += blockDim.x) {
+    const double2 h = f[x >> 5], l = f[nh + (x & 31)];
+    put(x, make_float2((float)(h.x * l.x - h.y * l.y), (float)(h.x * l.y + h.y * l.x)));
+  }
+}
+// SEARCH false: times the attenuation, inverse. true: common region, inverse; the first NR blocks of a
 // direction compute the step's ramps instead.
 template <int N, bool SEARCH>
 __global__ void __launch_bounds__(FCfg<N>::C* FCfg<N>::T, FCfg<N>::blocks(FCfg<N>::C* FCfg<N>::T, FCfg<N>::R))
     k_fit_cols(const ulonglong2* __restrict__ in, ulonglong2* __restrict__ out, const __grid_constant__ FitArgs A,
-               double dist, int RB) {
+               double dist) {
   using P = FCfg<N>;
   constexpr int T = P::T, C = P::C, E = P::E;
+  extern __shared__ ulonglong2 smp[];
+  static_assert((N / 32 + 32) * sizeof(double2) <= P::XC * sizeof(ulonglong2), "a ramp's factors fit the exchange buffer");
   const int lt = threadIdx.x, lane = lt % C, t = lt / C, a = blockIdx.y;
   if constexpr (SEARCH) {
-    if ((int)blockIdx.x < RB) {
+    if (blockIdx.x < NR) {  // fourierShift(kx, -ky) of every grid column and row
       const FitDir& d = A.dir[a];
-      float2* r = A.ramps + (size_t)a * (3 + NG) * N;
-      // x: the ramps of grid columns 2 and 7 and the step between columns; y: fourierShift(kx, -ky) of
-      // every grid row
-      for (int i = blockIdx.x * blockDim.x + lt; i < (3 + NG) * N; i += RB * blockDim.x) {
-        const int j = i / N, x = i % N;
-        r[(size_t)j * N + x] =
-            ramp_search(j == 0 ? d.kxs[2] : j == 1 ? d.kxs[7] : j == 2 ? d.kxs[5] - d.kxs[4] : -d.kys[j - 3], x, 1.0 / N);
+      float2* r = A.ramps + (size_t)a * NR * N;
+      const int j = blockIdx.x;
+      double2* f = reinterpret_cast<double2*>(smp);
+      if (j < NG) {
+        float* q = reinterpret_cast<float*>(r + (size_t)(j % (NG / 2)) * 2 * N) + j / (NG / 2);
+        ramp_search(d.kxs[j], N, f, [&](int x, float2 v) {
+          q[4 * x] = v.x;
+          q[4 * x + 2] = v.y;
+        });
+      } else {
+        ramp_search(-d.kys[j - NG], N, f, [&](int y, float2 v) { r[(size_t)j * N + y] = v; });
       }
       return;
     }
   }
-  const int x = (blockIdx.x - (SEARCH ? RB : 0)) * C + lane;
-  extern __shared__ ulonglong2 smp[];
+  const int x = (blockIdx.x - (SEARCH ? NR : 0)) * C + lane;
   const ulonglong2* ip = in + (size_t)a * N * N + x;
   cpair v[E];
 #pragma unroll
@@ -265,10 +282,10 @@ __global__ void __launch_bounds__(FCfg<N>::G* FCfg<N>::T, FCfg<N>::blocks(FCfg<N
 #pragma unroll
   for (int i = 0; i < E; i++) V[row + i * T] = p[i];
 }
-// Grid row sums: Q[j] = sum_x b1 conj(b0) exp(2 pi i kxs[j] x / N), and sum_x |b0|^2. The ten ramps come
-// from two of them and the step between neighbours (two further products at most); a thread's pixels
-// and the threads of equal lane are added in float, as the 32 partial sums of a warp-per-row
-// evaluation, then those in FP64. The transforms' 1/N^2 cancels against the norm.
+// Grid row sums: Q[j] = sum_x b1 conj(b0) exp(2 pi i kxs[j] x / N), two ramps at a time in packed
+// arithmetic, and sum_x |b0|^2. A thread's pixels and the threads of equal lane are added in float, as the
+// 32 partial sums of a warp-per-row evaluation, then those in FP64; the norm's float squares are added
+// exactly to 2^-45 (a sum of two floats), then in FP64. The transforms' 1/N^2 cancels against the norm.
 template <int N>
 __global__ void __launch_bounds__(FCfg<N>::G* FCfg<N>::T, FCfg<N>::blocks(FCfg<N>::G* FCfg<N>::T, FCfg<N>::E <= 8 ? 96 : 128))
     k_fit_rows(const ulonglong2* __restrict__ W, const __grid_constant__ FitArgs A) {
@@ -285,39 +302,55 @@ __global__ void __launch_bounds__(FCfg<N>::G* FCfg<N>::T, FCfg<N>::blocks(FCfg<N
     x[i] = cpair{u.x, u.y};
   }
   line_fft_pair<N, T, 1, true>(x, s, 0, t, g_stw + stw_offset(N, E));
-  const float2* r = A.ramps + (size_t)a * (3 + NG) * N + t;
-  float2 q[NG];
+  const ulonglong2* r = reinterpret_cast<const ulonglong2*>(A.ramps + (size_t)a * NR * N) + t;
+  cpair q[NG / 2];  // ramps j and j + NG/2
 #pragma unroll
-  for (int j = 0; j < NG; j++) q[j] = make_float2(0.f, 0.f);
-  float nrm = 0.f;
-  auto acc = [&](int j, float2 p) {
-    q[j].x += p.x;
-    q[j].y += p.y;
+  for (int j = 0; j < NG / 2; j++) q[j] = cp_zero();
+  float ns = 0.f, ne = 0.f;
+  auto add_norm = [&](float v) {
+    float s, z;
+    ff_two_sum(ns, v, s, z);
+    ns = s;
+    ne = __fadd_rn(ne, z);
   };
 #pragma unroll
   for (int i = 0; i < E; i++) {
     float2 b0, b1;
     cp_split(x[i], b0, b1);
-    nrm += b0.x * b0.x + b0.y * b0.y;
-    const float2 p = cmulc(b1, b0), d = __ldg(r + 2 * N + i * T);
+    add_norm(__fmul_rn(b0.x, b0.x));
+    add_norm(__fmul_rn(b0.y, b0.y));
+    const wpair p = w_dup(cmulc(b1, b0));
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const float2 c = cmul(p, __ldg(r + h * N + i * T)), u1 = cmul(c, d), l1 = cmulc(c, d);
-      acc(5 * h + 2, c);
-      acc(5 * h + 3, u1);
-      acc(5 * h + 4, cmul(u1, d));
-      acc(5 * h + 1, l1);
-      acc(5 * h, cmulc(l1, d));
+    for (int j = 0; j < NG / 2; j++) {
+      const ulonglong2 w = __ldg(r + (size_t)j * N + i * T);
+      q[j] = cadd(q[j], cmul(cpair{w.x, w.y}, p));
     }
   }
   float* part = reinterpret_cast<float*>(smp + P::G * P::XS) + (size_t)g * NV * (T + 1);  // [value][T + 1]
 #pragma unroll
-  for (int j = 0; j < NG; j++) {
-    part[(2 * j) * (T + 1) + t] = q[j].x;
-    part[(2 * j + 1) * (T + 1) + t] = q[j].y;
+  for (int j = 0; j < NG / 2; j++) {
+    float2 u, v;
+    cp_split(q[j], u, v);
+    part[(2 * j) * (T + 1) + t] = u.x;
+    part[(2 * j + 1) * (T + 1) + t] = u.y;
+    part[(2 * j + NG) * (T + 1) + t] = v.x;
+    part[(2 * j + NG + 1) * (T + 1) + t] = v.y;
   }
-  part[2 * NG * (T + 1) + t] = nrm;
+  constexpr int NWP = (T + 31) / 32;  // warps per row
+  __shared__ double norm[P::G][NWP];
+#pragma unroll
+  for (int o = P::PT / 2; o > 0; o >>= 1) {  // PT lanes: the warp, or the row's share of it
+    const float s = __shfl_xor_sync(0xffffffffu, ns, o), z = __shfl_xor_sync(0xffffffffu, ne, o);
+    add_norm(s);
+    ne = __fadd_rn(ne, z);
+  }
+  if (t % P::PT == 0) norm[g][t / P::PT] = (double)ns + (double)ne;
   __syncthreads();
+  if (t == 0) {
+    double d = norm[g][0];
+    for (int k = 1; k < NWP; k++) d += norm[g][k];
+    A.n2[(size_t)a * N + y] = d;
+  }
   // four threads per value (neighbours in a warp), an eighth of the PT partial sums at a time
   for (int k = t; k < 4 * NV; k += T) {
     const int v = k / 4, h = k % 4;
@@ -333,10 +366,7 @@ __global__ void __launch_bounds__(FCfg<N>::G* FCfg<N>::T, FCfg<N>::blocks(FCfg<N
     const unsigned four = 0xfu << (threadIdx.x & 28);  // enter together: T and 4 * NV are multiples of 4
     d += __shfl_xor_sync(four, d, 1);
     d += __shfl_xor_sync(four, d, 2);
-    if (h == 0) {
-      if (v == 2 * NG) A.n2[(size_t)a * N + y] = d;
-      else reinterpret_cast<double*>(A.Q + ((size_t)a * NG + v / 2) * N + y)[v & 1] = d;
-    }
+    if (h == 0) reinterpret_cast<double*>(A.Q + ((size_t)a * NG + v / 2) * N + y)[v & 1] = d;
   }
 }
 
@@ -492,7 +522,7 @@ __global__ void __launch_bounds__(128) k_fit_grid(const __grid_constant__ FitArg
   const int jx = g % NG, jy = g / NG;
   FitDir& d = A.dir[a];
   const double2* Q = A.Q + ((size_t)a * NG + jx) * n;
-  const float2* ty = A.ramps + ((size_t)a * (3 + NG) + 3 + jy) * n;
+  const float2* ty = A.ramps + ((size_t)a * NR + NG + jy) * n;
   double re = 0, im = 0;
   for (int y = i; y < n; y += NT) {
     const double2 q = Q[y];
@@ -570,7 +600,7 @@ __global__ void __launch_bounds__(128) k_fit_region(const ulonglong2* __restrict
   const int x = blockIdx.x * 128 + threadIdx.x, y = blockIdx.y, a = blockIdx.z;
   if (x >= N) return;
   const FitDir& d = A.dir[a];
-  if (y < 2) A.ramps[((size_t)a * (3 + NG) + 3 * y) * N + x] = ramp_at(y == 0 ? d.kxs[0] : -d.kys[0], x, N);
+  if (y < 2) A.ramps[((size_t)a * NR + NG * y) * N + x] = ramp_at(y == 0 ? d.kxs[0] : -d.kys[0], x, N);
   const size_t n = (size_t)N * N, i = (size_t)y * N + x;
   const Region R = region_of<N>(d.cp, dist);
   const float2 f = p_unpack(common_factor<N>(A, R, x, y));
@@ -607,7 +637,7 @@ __global__ void __launch_bounds__(128) k_fit_peak_sum(const __grid_constant__ Fi
   FitDir& d = A.dir[a];
   double* res = A.results + 8 * a;
   const double2* Q = A.Q + (size_t)a * NG * n;
-  const float2* ty = A.ramps + ((size_t)a * (3 + NG) + 3) * n;
+  const float2* ty = A.ramps + ((size_t)a * NR + NG) * n;
   double v[3] = {0, 0, 0};
   for (int y = i; y < n; y += NT) {
     const double2 q = Q[y];
@@ -674,17 +704,17 @@ int fit_run(const SpecIn& spec, const MixCoef& fitted, const MixCoef* other, int
     attr = true;
   }
   const dim3 gr(N / P::G, nA), gc(N / P::C, nA);
-  const int nr = P::G * P::T, nc = P::C * P::T, RB = std::max(1, (3 + NG) * N / (4 * nc));
+  const int nr = P::G * P::T, nc = P::C * P::T;
   const double dist = 0.15;
   const dim3 gsep(std::max(1, 8 * ctx().num_sms / nA), nA);
   k_fit_separate<<<gsep, 256, 0, st>>>(spec, fitted, nP, (size_t)N * N, B.S);
   if (other) k_fit_separate<<<gsep, 256, 0, st>>>(spec, *other, nP, (size_t)N * N, B.L);
-  k_fit_cols<N, false><<<gc, nc, sm_col, st>>>(B.S, B.W, B.A, dist, 0);
+  k_fit_cols<N, false><<<gc, nc, sm_col, st>>>(B.S, B.W, B.A, dist);
   k_fit_rows_product<N><<<gr, nr, sm_row, st>>>(B.W, B.V);
   k_fit_peak<N><<<dim3(PB, nA), nc, sm_peak, st>>>(B.V, r2_lim, B.A);
   k_fit_start<<<nA, 256, 0, st>>>(B.A, PB, N, dist);
   for (int step = 0; step < 3; step++) {
-    k_fit_cols<N, true><<<dim3(RB + N / P::C, nA), nc, sm_col, st>>>(B.S, B.W, B.A, dist, RB);
+    k_fit_cols<N, true><<<dim3(NR + N / P::C, nA), nc, sm_col, st>>>(B.S, B.W, B.A, dist);
     k_fit_rows<N><<<gr, nr, sm_q, st>>>(B.W, B.A);
     k_fit_grid<<<dim3(NG * NG, nA), 128, 0, st>>>(B.A, N, step, dist, task[0].scale);
   }
@@ -696,7 +726,7 @@ int fit_run(const SpecIn& spec, const MixCoef& fitted, const MixCoef* other, int
     k_fit_norm<<<dim3(N / 8, nA), 256, 0, st>>>(B.V, N, B.A);
     for (int a = 0; a < nA; a++)
       k_corr_rows<1><<<N / CORR_ROWS_PER_BLOCK, 32 * CORR_ROWS_PER_BLOCK, 0, st>>>(
-          B.V + (size_t)(2 * a) * N * N, B.V + (size_t)(2 * a + 1) * N * N, B.A.ramps + (size_t)a * (3 + NG) * N, N, 1,
+          B.V + (size_t)(2 * a) * N * N, B.V + (size_t)(2 * a + 1) * N * N, B.A.ramps + (size_t)a * NR * N, N, 1,
           B.A.Q + (size_t)a * NG * N);
     k_fit_peak_sum<<<nA, 128, 0, st>>>(B.A, N, task[k].out, dist, k + 1 < ntask ? task[k + 1].scale : 0.);
   }
@@ -771,7 +801,7 @@ int fit_pairs(const fsim_sim_param* p, const FitSource& src, int fit_band, doubl
   // an estimated OTF's table ends before the measured bands
   const size_t o_fx = al(offsetof(OtfTable, mvals)), o_fy = o_fx + sizeof(double) * N, consts = al(o_fy + sizeof(float) * N);
   const size_t sizes[] = {plane, other >= 0 ? plane : 0, plane, std::max(spectra, work) - plane, al(sizeof(float) * n),
-                          al(sizeof(float) * n), al(sizeof(float2) * (3 + NG) * N * nA), al(sizeof(double2) * NG * N * nA),
+                          al(sizeof(float) * n), al(sizeof(float2) * NR * N * nA), al(sizeof(double2) * NG * N * nA),
                           al(sizeof(double) * N * nA), al(sizeof(float) * N * nA), al(sizeof(int) * N * nA),
                           al(sizeof(FitDir) * nA), al(sizeof(double) * 8 * nA), consts};
   size_t total = 0;
