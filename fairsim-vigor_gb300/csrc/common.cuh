@@ -21,10 +21,15 @@ cudaError_t dev_alloc(T** p, size_t bytes) {
   return dev_alloc(reinterpret_cast<void**>(p), bytes);
 }
 // Stream-ordered scratch (freed with cudaFreeAsync) from a pool that keeps up to 512 MiB
-// between calls: without it every call maps and unmaps its memory. The pool serves any number of
-// threads and streams (the runtime orders reuse), and its idle memory is returned when another
-// allocation of the library would fail.
+// between calls: without it every call maps and unmaps its memory (a fit of 1024^2, waited for: 730 us,
+// 1214 without). The pool serves any number of threads and streams (the runtime orders reuse). Its idle
+// memory is given back when another allocation of the library would fail, when the server needs it for
+// slots, when a plan is destroyed or a server closed, and by fsim_sync while less than hbm_headroom() of
+// the device is free.
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t st);
+bool release_idle_scratch();  // false when there is none
+// device memory left to other users of the GPU
+size_t hbm_headroom(size_t total);
 template <class T>
 cudaError_t dev_alloc_async(T** p, size_t bytes, cudaStream_t st) {
   return dev_alloc_async(reinterpret_cast<void**>(p), bytes, st);

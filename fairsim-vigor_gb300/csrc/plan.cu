@@ -346,6 +346,7 @@ int fsim_plan_destroy(fsim_plan* plan) {
   if (plan->h_ws) cudaFree(plan->h_ws);
   if (plan->h_io) cudaFree(plan->h_io);
   if (plan->h_job) cudaFreeHost(plan->h_job);
+  release_idle_scratch();
   delete plan;
   return FSIM_OK;
 }

@@ -1,4 +1,5 @@
 // Library runtime: error state, device/stream context, FFT twiddle tables.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
@@ -46,6 +47,22 @@ static bool trim_pool() {
   if (!g_pool) return false;
   (void)cudaGetLastError();  // the failed allocation's
   return cudaDeviceSynchronize() == cudaSuccess && cudaMemPoolTrimTo(g_pool, 0) == cudaSuccess;
+}
+
+// bytes the pool holds and nobody uses
+static size_t pool_idle() {
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  unsigned long long held = 0, used = 0;
+  if (!g_pool || cudaMemPoolGetAttribute(g_pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+      cudaMemPoolGetAttribute(g_pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return held > used ? (size_t)(held - used) : 0;
+}
+size_t hbm_headroom(size_t total) { return std::max(total / 16, (size_t)1 << 30); }
+bool release_idle_scratch() {
+  if (pool_idle() == 0) return false;
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  return cudaMemPoolTrimTo(g_pool, 0) == cudaSuccess;
 }
 
 cudaError_t dev_alloc(void** p, size_t bytes) {
@@ -188,6 +205,10 @@ int fsim_sync(void) {
   int rc = fsim::ensure_init();
   if (rc) return rc;
   FSIM_CUDA(cudaDeviceSynchronize());
+  size_t free_b = 0, total_b = 0;  // (a query takes longer than the wait: only for memory worth it)
+  if (fsim::pool_idle() >= (size_t)16 << 20 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+      free_b < fsim::hbm_headroom(total_b))
+    fsim::release_idle_scratch();
   return FSIM_OK;
 }
 

@@ -392,9 +392,6 @@ int fsim_serve_open(fsim_server** out, const fsim_serve_config* cfg, const fsim_
 
 }  // extern "C"
 
-// Device memory left to other users of the GPU when slots are sized from its free HBM.
-static size_t hbm_headroom(size_t total) { return std::max(total / 16, (size_t)1 << 30); }
-
 // One slot of class c: pinned host staging and device buffers; false when an allocation fails
 // (whatever was allocated is released).
 static bool alloc_slot(const fsim_server::SlotClass& c, fsim_server::Slot* sl) {
@@ -452,7 +449,9 @@ static void grow_slots(fsim_server* s) {
     }
     if (c < 0) return;
     const auto& sc = s->cls[c];  // the class list is fixed after open
-    if (slot_room(s, slot_bytes_now) < sc.raw_bytes + sc.out_bytes) return;
+    const size_t need = sc.raw_bytes + sc.out_bytes;
+    // the library's own idle scratch counts as free: it is given back where a slot needs it
+    if (slot_room(s, slot_bytes_now) < need && !(release_idle_scratch() && slot_room(s, slot_bytes_now) >= need)) return;
     fsim_server::Slot sl;
     if (!alloc_slot(sc, &sl)) return;
     sl.cls = c;

@@ -47,7 +47,10 @@ extern "C" {
 /* ---- library ------------------------------------------------------------------- */
 const char* fsim_last_error(void);
 int fsim_init(int device);               /* select device, upload FFT twiddle tables */
-int fsim_sync(void);                     /* AccelVectorFactory.nativeSync (cudaDeviceSynchronize) */
+/* AccelVectorFactory.nativeSync (cudaDeviceSynchronize). Calls that need scratch keep up to 512 MiB of
+ * it for the next one; it is given back here while device memory is scarce (less than 1/16 free), and
+ * whenever a plan is destroyed or a server closed. */
+int fsim_sync(void);
 int fsim_version(void);
 int fsim_set_stream(void* stream);       /* stream used by the vector API (NULL = own stream) */
 
