@@ -24,7 +24,9 @@ struct LinePlan {
   static constexpr int E = (L % 3 == 0) ? 12 : (L >= 64 ? 8 : 4);
   static constexpr int T = L / E;
   static constexpr int G = T >= 128 ? 1 : 128 / T;                     // row pairs per block
-  static constexpr int CP = T >= 512 ? 1 : (T >= 256 ? 2 : (T >= 32 ? 4 : 8));  // column pairs per block
+  // column pairs per block; two at the longest lines although one block then fills an SM: one pair reads 16
+  // bytes of every row, half a sector (4096^2: 176 us, 141 with two)
+  static constexpr int CP = T >= 256 ? 2 : (T >= 32 ? 4 : 8);
   static constexpr int R = E <= 8 ? 64 : 128;                          // registers per thread
   static constexpr int blocks(int threads) { return 65536 / (threads * R) > 0 ? 65536 / (threads * R) : 1; }
 };
