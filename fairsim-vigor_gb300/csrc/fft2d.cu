@@ -148,43 +148,8 @@ static bool len_ok(int L) {
 
 bool fft2d_supported(int w, int h) { return len_ok(w) && len_ok(h); }
 
-static int rows_dispatch(int L, bool inv, float2* d, int nrows, int batch, size_t stride, float scale, cudaStream_t st) {
-  switch (L) {
-#define CASE(n)                                                                          \
-  case n:                                                                                \
-    return inv ? launch_rows<n, true>(d, nrows, batch, stride, scale, st)               \
-               : launch_rows<n, false>(d, nrows, batch, stride, scale, st);
-    FSIM_FFT_LENGTHS(CASE)
-#undef CASE
-  }
-  set_error("unsupported FFT length %d", L);
-  return FSIM_EINVAL;
-}
-static int cols_dispatch(int L, bool inv, float2* d, int ncols, int batch, size_t stride, float scale, cudaStream_t st) {
-  switch (L) {
-#define CASE(n)                                                                          \
-  case n:                                                                                \
-    return inv ? launch_cols<n, true>(d, ncols, batch, stride, scale, st)               \
-               : launch_cols<n, false>(d, ncols, batch, stride, scale, st);
-    FSIM_FFT_LENGTHS(CASE)
-#undef CASE
-  }
-  set_error("unsupported FFT length %d", L);
-  return FSIM_EINVAL;
-}
-
-int fft2d_device(float2* data, int w, int h, bool inverse, cudaStream_t stream, int batch) {
-  FSIM_REQUIRE(fft2d_supported(w, h), FSIM_EINVAL,
-               "fft2d: unsupported size %d x %d (lengths 2^k in 32..4096 and 3*2^k in 48..3072)", w, h);
-  size_t stride = (size_t)w * h;
-  int rc = rows_dispatch(w, inverse, data, h, batch, stride, 1.f, stream);
-  if (rc) return rc;
-  float scale = inverse ? (float)(1.0 / ((double)w * (double)h)) : 1.f;
-  return cols_dispatch(h, inverse, data, w, batch, stride, scale, stream);
-}
-
 // ---- the same transform one line at a time ----------------------------------------------------
-// The parameter fit's spectra and getPeak's inverse transforms keep this plan (16 elements per
+// For small arrays (lines_faster), and in the fit: the parameter fit's spectra and getPeak's inverse transforms keep this plan (16 elements per
 // thread at 1024 and beyond): the fitted modulations are reported in double, and another order
 // of the same roundings moves them by 5e-9 relative, so callers that compare fits would see it.
 template <int L>
@@ -280,35 +245,130 @@ constexpr auto cols1_kernel() {
   if constexpr (LineOne<L>::E <= 8) return k_fft1_cols<L, INV>;
   else return k_fft1_cols_wide<L, INV>;
 }
-template <int L, bool INV, bool RAW>
-static int launch_lines(float2* d, int batch, const RawFade& rf, cudaStream_t st) {
+// In small arrays the pairs' half as many threads and, at 1024 and beyond, one exchange more show as
+// latency: 64^2 3.6 us, 3.3 by lines, 256^2 5.4 and 5.2, 1024^2 11.0 and 10.1, 256 x 1024 8.5 and 7.7, 512 x 2048 11.2
+// and 10.3; 4 x 512^2 take 9.0 either way, 2 x 1024^2 16.0 and 17.4. Lengths 3*2^k are faster in pairs at
+// every size (768^2 9.5, 11.4 by lines).
+static bool lines_faster(int w, int h, int batch) {
+  auto ok = [](int L) { return (L & (L - 1)) == 0 && L >= 64; };
+  return ok(w) && ok(h) && (size_t)w * h * batch <= (size_t)(std::max(w, h) >= 1024 ? 1 << 20 : 1 << 19);
+}
+template <int L, bool INV>
+static int line_rows(float2* d, int nrows, int batch, size_t stride, cudaStream_t st) {
   using P = LineOne<L>;
-  const size_t sm_r = sizeof(float2) * (size_t)P::G * smem_line_elems(L, 1), sm_c = sizeof(float2) * smem_line_elems(L, P::C);
+  const size_t smem = sizeof(float2) * (size_t)P::G * smem_line_elems(L, 1);
+  static bool attr = false;
+  if (!attr) {
+    FSIM_CUDA(cudaFuncSetAttribute(k_fft1_rows<L, INV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr = true;
+  }
+  k_fft1_rows<L, INV, false><<<dim3(div_up(nrows, P::G), batch), P::G * P::T, smem, st>>>(d, nrows, stride, RawFade{});
+  FSIM_CHECK_LAUNCH();
+  return FSIM_OK;
+}
+template <int L, bool INV>
+static int line_cols(float2* d, int ncols, int batch, size_t stride, float scale, cudaStream_t st) {
+  using P = LineOne<L>;
+  const size_t smem = sizeof(float2) * smem_line_elems(L, P::C);
   auto cols = cols1_kernel<L, INV>();
   static bool attr = false;
   if (!attr) {
-    FSIM_CUDA(cudaFuncSetAttribute(k_fft1_rows<L, INV, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_r));
-    FSIM_CUDA(cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_c));
+    FSIM_CUDA(cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr = true;
   }
-  const size_t stride = (size_t)L * L;
-  k_fft1_rows<L, INV, RAW><<<dim3(div_up(L, P::G), batch), P::G * P::T, sm_r, st>>>(d, L, stride, rf);
-  cols<<<dim3(div_up(L, P::C), batch), P::C * P::T, sm_c, st>>>(d, L, stride,
-                                                              INV ? (float)(1.0 / ((double)L * (double)L)) : 1.f);
+  cols<<<dim3(div_up(ncols, P::C), batch), P::C * P::T, smem, st>>>(d, ncols, stride, scale);
   FSIM_CHECK_LAUNCH();
   return FSIM_OK;
+}
+static int lines_2d(float2* d, int w, int h, bool inv, cudaStream_t st, int batch) {
+  const size_t stride = (size_t)w * h;
+  const float scale = inv ? (float)(1.0 / ((double)w * (double)h)) : 1.f;
+  int rc = FSIM_EINVAL;
+#define FSIM_LINE_LENGTHS(X) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
+  switch (w) {
+#define CASE(n) \
+  case n: rc = inv ? line_rows<n, true>(d, h, batch, stride, st) : line_rows<n, false>(d, h, batch, stride, st); break;
+    FSIM_LINE_LENGTHS(CASE)
+#undef CASE
+  }
+  if (rc) return rc;
+  switch (h) {
+#define CASE(n) \
+  case n:       \
+    return inv ? line_cols<n, true>(d, w, batch, stride, scale, st) : line_cols<n, false>(d, w, batch, stride, scale, st);
+    FSIM_LINE_LENGTHS(CASE)
+#undef CASE
+  }
+  return FSIM_EINVAL;
+}
+template <int L>
+static int raw_rows_launch(float2* d, int batch, const RawFade& rf, cudaStream_t st) {
+  using P = LineOne<L>;
+  const size_t smem = sizeof(float2) * (size_t)P::G * smem_line_elems(L, 1);
+  static bool attr = false;
+  if (!attr) {
+    FSIM_CUDA(cudaFuncSetAttribute(k_fft1_rows<L, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr = true;
+  }
+  k_fft1_rows<L, false, true><<<dim3(div_up(L, P::G), batch), P::G * P::T, smem, st>>>(d, L, (size_t)L * L, rf);
+  FSIM_CHECK_LAUNCH();
+  return FSIM_OK;
+}
+template <int L>
+static int fit_lines(float2* d, int batch, const RawFade* raw, cudaStream_t st) {
+  const size_t stride = (size_t)L * L;
+  int rc = raw ? raw_rows_launch<L>(d, batch, *raw, st) : line_rows<L, true>(d, L, batch, stride, st);
+  if (rc) return rc;
+  return raw ? line_cols<L, false>(d, L, batch, stride, 1.f, st)
+             : line_cols<L, true>(d, L, batch, stride, (float)(1.0 / ((double)L * (double)L)), st);
 }
 #define FSIM_LINE_SIZES(X) X(128) X(256) X(384) X(512) X(768) X(1024) X(2048)
 int fft2d_lines_device(float2* data, int n, cudaStream_t st, int batch, const RawFade* raw) {
   switch (n) {
 #define CASE(v) \
   case v:       \
-    return raw ? launch_lines<v, false, true>(data, batch, *raw, st) : launch_lines<v, true, false>(data, batch, RawFade{}, st);
+    return fit_lines<v>(data, batch, raw, st);
     FSIM_LINE_SIZES(CASE)
 #undef CASE
   }
   set_error("line-by-line FFT: unsupported size %d", n);
   return FSIM_EINVAL;
+}
+
+static int rows_dispatch(int L, bool inv, float2* d, int nrows, int batch, size_t stride, float scale, cudaStream_t st) {
+  switch (L) {
+#define CASE(n)                                                                          \
+  case n:                                                                                \
+    return inv ? launch_rows<n, true>(d, nrows, batch, stride, scale, st)               \
+               : launch_rows<n, false>(d, nrows, batch, stride, scale, st);
+    FSIM_FFT_LENGTHS(CASE)
+#undef CASE
+  }
+  set_error("unsupported FFT length %d", L);
+  return FSIM_EINVAL;
+}
+static int cols_dispatch(int L, bool inv, float2* d, int ncols, int batch, size_t stride, float scale, cudaStream_t st) {
+  switch (L) {
+#define CASE(n)                                                                          \
+  case n:                                                                                \
+    return inv ? launch_cols<n, true>(d, ncols, batch, stride, scale, st)               \
+               : launch_cols<n, false>(d, ncols, batch, stride, scale, st);
+    FSIM_FFT_LENGTHS(CASE)
+#undef CASE
+  }
+  set_error("unsupported FFT length %d", L);
+  return FSIM_EINVAL;
+}
+
+int fft2d_device(float2* data, int w, int h, bool inverse, cudaStream_t stream, int batch) {
+  FSIM_REQUIRE(fft2d_supported(w, h), FSIM_EINVAL,
+               "fft2d: unsupported size %d x %d (lengths 2^k in 32..4096 and 3*2^k in 48..3072)", w, h);
+  if (lines_faster(w, h, batch)) return lines_2d(data, w, h, inverse, stream, batch);
+  size_t stride = (size_t)w * h;
+  int rc = rows_dispatch(w, inverse, data, h, batch, stride, 1.f, stream);
+  if (rc) return rc;
+  float scale = inverse ? (float)(1.0 / ((double)w * (double)h)) : 1.f;
+  return cols_dispatch(h, inverse, data, w, batch, stride, scale, stream);
 }
 
 }  // namespace fsim
