@@ -591,7 +591,6 @@ void Plan::fill_job_live(JobDesc& j, const void* raw, float* out, float* wf, cha
   j.nA = prm.nr_dirs;
   j.nP = prm.nr_phases;
   j.nC = nC;
-  j.status = ctx().status;
   j.nWin = nwin;
   j.bgr = 0.f;
   j.damp = d_damp;

@@ -344,7 +344,6 @@ void Plan::fill_job(JobDesc& j, const void* raw, float* out, float* wf, float* f
   j.nP = prm.nr_phases;
   j.nC = nC;
   j.nWin = nwin;
-  j.status = ctx().status;
   j.cmask = otf_measured(&prm) ? 1 : 0;
   j.edge = d_edge;
   j.clip = clip_scale;

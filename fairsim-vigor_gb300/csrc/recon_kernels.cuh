@@ -894,9 +894,10 @@ __host__ inline int size_slot(int n) {
   return -1;
 }
 
-// variant lists: pass A (and G) elements/thread {E0, E1}; passes B1 and B2, each on its own,
-// (elements, columns per block) {(E0,4), (E0,2), (E1,4), (E1,2)} with E0 = 8, E1 = 16
-// (3*2^k sizes: 12, 24). The extremes (N <= 128, N >= 2048) have one variant.
+// variant lists: pass A (and G) elements/thread {E0, E1}; passes B1 (long batches: the form of dependent
+// launches has one variant) and B2, each on its own, (elements, columns per block) {(E0,4), (E0,2),
+// (E1,4), (E1,2)} with E0 = 8, E1 = 16 (3*2^k sizes: 12, 24). The extremes (N <= 128, N >= 2048) have
+// one variant.
 template <int N>
 int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int maxWin, bool scale_clip, int kinds,
                    bool alone, cudaStream_t st) {
