@@ -381,6 +381,7 @@ struct PassB1 {
   static constexpr int XS = pair_elems(N, CP);
   static constexpr size_t SMEM = sizeof(ulonglong2) * (size_t)XS;
   static constexpr int MINB = pair_min_blocks(NT, P::EN, 80);
+  static constexpr bool BYJOB = P::EN > 8 && NT >= 128;  // grid order of k_pass_b01
 };
 // Row yl of window columns xl and xl + 1 of a component (col: the position of its first row in
 // the component-by-component window layout), times their masks, to Tw.
@@ -596,15 +597,16 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
 }
 // Band 0 and the pairs in one launch: the form of dependent launches, whose blocks all wait for pass A
 // (and G) before they read what it wrote, and of the jobs with edge weights (EDGE). Band 0, the shorter
-// work, comes last: of each job at 3*2^k lengths, of all jobs at 2^k (4 x 1024^2 359 us, 364 job by job, but 4 x
-// 768^2 230 job by job and 242 the other way). In long batches the two kernels are faster: band 0 by itself
+// work, comes last of all jobs (4 x 1024^2 358 us, 366 with it last of each job; 7 x 384^2 three-band 197, 202), but
+// job by job where 12 elements per thread make blocks of 128 threads (4 x 768^2 231 us, 240 the other way): four
+// of those fill an SM. In long batches the two kernels are faster: band 0 by itself
 // needs fewer registers (16 x 512^2 306 us, 309 in one).
 template <int N, int ENV, int CBV, bool CM, bool EDGE>
 __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
     k_pass_b01(const JobDesc* __restrict__ jobs) {
   using P = Cfg<N, ENV, CBV>;
   using PB = PassB1<N, ENV, CBV>;
-  constexpr bool BYJOB = N % 3 == 0;
+  constexpr bool BYJOB = PB::BYJOB;
   const int lt = threadIdx.x, x0 = blockIdx.x * P::CB;
   const int c = BYJOB ? blockIdx.y : blockIdx.z, comp = c + 1 < (int)(BYJOB ? gridDim.y : gridDim.z) ? c + 1 : 0;
   __shared__ JobDesc J;
@@ -844,7 +846,7 @@ static int launch_b_one(bool dep, const JobDesc* d_jobs, int njobs, int maxA, in
   int rc = grant_smem(k_pass_b01<N, ENB, CBB, CM, EDGE>, PB::SMEM, attr);
   if (rc) return rc;
   const int gx = (maxWin + CB - 1) / CB, comps = 1 + maxA * maxPair;
-  FSIM_CUDA(launch_pass(dep, k_pass_b01<N, ENB, CBB, CM, EDGE>, N % 3 == 0 ? dim3(gx, comps, njobs) : dim3(gx, njobs, comps),
+  FSIM_CUDA(launch_pass(dep, k_pass_b01<N, ENB, CBB, CM, EDGE>, PB::BYJOB ? dim3(gx, comps, njobs) : dim3(gx, njobs, comps),
                         PB::NT, PB::SMEM, st, d_jobs));
   return FSIM_OK;
 }
