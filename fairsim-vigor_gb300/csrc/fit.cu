@@ -234,8 +234,10 @@ __global__ void __launch_bounds__(FCfg<N>::C* FCfg<N>::T, FCfg<N>::blocks(FCfg<N
     const Region R = region_of<N>(A.dir[a].cp, dist);
 #pragma unroll
     for (int i = 0; i < E; i++) {
-      const f32x2 f = common_factor<N>(A, R, x, t + i * T);
-      v[i] = cpair{p_mul(v[i].re, f), p_mul(v[i].im, f)};
+      const float2 f = p_unpack(common_factor<N>(A, R, x, t + i * T)), re = p_unpack(v[i].re), im = p_unpack(v[i].im);
+      // (a bin that is cut is 0, whatever it held)
+      v[i] = cpair{p_pack(f.x == 0.f ? 0.f : re.x * f.x, f.y == 0.f ? 0.f : re.y * f.y),
+                   p_pack(f.x == 0.f ? 0.f : im.x * f.x, f.y == 0.f ? 0.f : im.y * f.y)};
     }
   } else {
 #pragma unroll
