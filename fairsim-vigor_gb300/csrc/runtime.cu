@@ -1,6 +1,7 @@
 // Library runtime: error state, device/stream context, FFT twiddle tables.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <mutex>
@@ -59,6 +60,16 @@ static size_t pool_idle() {
   return held > used ? (size_t)(held - used) : 0;
 }
 size_t hbm_headroom(size_t total) { return std::max(total / 16, (size_t)1 << 30); }
+// The query of the free memory takes 25 us: at most once in 10 ms, and only for memory worth it.
+static void release_scratch_if_scarce() {
+  static std::atomic<long long> last{0};
+  const long long now = std::chrono::duration_cast<std::chrono::milliseconds>(
+                            std::chrono::steady_clock::now().time_since_epoch()).count();
+  if (now - last.load(std::memory_order_relaxed) < 10 || pool_idle() < (size_t)16 << 20) return;
+  last.store(now, std::memory_order_relaxed);
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < hbm_headroom(total_b)) release_idle_scratch();
+}
 bool release_idle_scratch() {
   if (pool_idle() == 0) return false;
   std::lock_guard<std::mutex> g(g_pool_mu);
@@ -205,10 +216,7 @@ int fsim_sync(void) {
   int rc = fsim::ensure_init();
   if (rc) return rc;
   FSIM_CUDA(cudaDeviceSynchronize());
-  size_t free_b = 0, total_b = 0;  // (a query takes longer than the wait: only for memory worth it)
-  if (fsim::pool_idle() >= (size_t)16 << 20 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-      free_b < fsim::hbm_headroom(total_b))
-    fsim::release_idle_scratch();
+  fsim::release_scratch_if_scarce();
   return FSIM_OK;
 }
 
