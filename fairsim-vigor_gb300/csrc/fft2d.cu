@@ -3,6 +3,7 @@
 //   pass 1: rows    - two adjacent rows per thread group, coalesced row loads;
 //   pass 2: columns - pairs of adjacent columns, CP pairs interleaved in shared memory so that
 //           every global access of a row moves CP * 16 contiguous bytes.
+// Small power-of-two arrays run line by line instead (lines_faster, below).
 // Each pass reads and writes the array once (16 bytes per complex element per pass): 16 planes of
 // 1024^2 in 112 us on GB300, 134 one line at a time (79 at the rate of a plain copy); the column
 // pass, with 64-byte pieces of each row, is the slower one.

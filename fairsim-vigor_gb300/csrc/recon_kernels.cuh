@@ -599,8 +599,8 @@ __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::
 // (and G) before they read what it wrote, and of the jobs with edge weights (EDGE). Band 0, the shorter
 // work, comes last of all jobs (4 x 1024^2 358 us, 366 with it last of each job; 7 x 384^2 three-band 197, 202), but
 // job by job where 12 elements per thread make blocks of 128 threads (4 x 768^2 231 us, 240 the other way): four
-// of those fill an SM. In long batches the two kernels are faster: band 0 by itself
-// needs fewer registers (16 x 512^2 306 us, 309 in one).
+// of those fill an SM. As ordinary launches the two kernels are faster: band 0 by itself needs fewer
+// registers (16 x 512^2 306 us, 309 in one).
 template <int N, int ENV, int CBV, bool CM, bool EDGE>
 __global__ void __launch_bounds__(PassB1<N, ENV, CBV>::NT, PassB1<N, ENV, CBV>::MINB)
     k_pass_b01(const JobDesc* __restrict__ jobs) {
@@ -909,9 +909,11 @@ int launch_offline(const JobDesc* d_jobs, int njobs, int maxA, int maxPair, int 
   constexpr int CBX = N >= 2048 ? 2 : 4;
   const int k = size_slot(N);
   const int va = single ? 0 : g_var_a[k], vb1 = single ? 0 : g_var_b[k], vb2 = single ? 0 : g_var_b2[k];
-  // Passes as dependent launches while a batch is short: one 256^2 stack 46.8 -> 34.4 us, 8 x 512^2
-  // 186 -> 177, 16 x 512^2 (16k blocks of pass A) 336 -> 328, but 64 x 512^2 1183 -> 1195 us, and a batch of
-  // several size classes, whose waiting blocks take the room of another class's passes, 3% longer.
+  // Passes as dependent launches while a batch is short (as graphs, without and with: one 256^2 stack 36.9
+  // and 30.7 us, 4 x 512^2 101 and 93, 8 x 512^2 167 and 160), but not in a batch of several size classes,
+  // whose waiting blocks take the room of another class's passes (3% longer). The line was drawn while
+  // pass B was two dependent launches, when 64 x 512^2 took 1183 us without and 1195 with; as one launch,
+  // longer batches gain too (16 x 512^2 307 and 297, 64 x 512^2 1100 and 1092).
   const bool dep = alone && (long long)(N / PassA<N, E0>::RB) * (maxA + 1) * njobs <= 64LL * ctx().num_sms;
   cudaEvent_t* ev = profile_events();
   if (ev) cudaEventRecord(ev[0], st);

@@ -268,8 +268,10 @@ int fsim_recon_batch_host(const fsim_host_job* jobs, int n_jobs, int chunk);
  * with the classes on parallel branches. Replays
  * (fsim_batch_graph_launch) reconstruct the same jobs' current raw buffers into the same
  * outputs. Plans, raw/out buffers and the workspace must stay allocated while the graph
- * exists; fsim_plan_update keeps a plan's table addresses, so replays pick up new
- * parameters. n_kernels: kernel launches per replay. */
+ * exists; replays pick up what fsim_plan_update gives a plan: its tables keep their addresses,
+ * and where an update changes what the record holds of the plan (a larger window, OTF supports
+ * that come to reach the output's Nyquist lines) the next launch records the batch again.
+ * n_kernels: kernel launches per replay. */
 typedef struct fsim_batch_graph fsim_batch_graph;
 int fsim_batch_graph_create(fsim_batch_graph** out, const fsim_job* jobs, int n_jobs, void* workspace,
                             size_t workspace_bytes, void* stream);

@@ -1,6 +1,6 @@
-"""The 2D FFT on both sides of the size where it goes from single lines to line pairs (powers of two:
-2^19 elements, 2^20 with lines of 1024 and beyond), at the shortest and longest lines, and 4096-point columns; 1e-6 relative L2 against
-a 64-bit FFT: about 2^-24 per level of the transform."""
+"""The 2D FFT on both sides of the size where it goes from single lines to line pairs (powers of
+two: 2^19 elements, 2^20 with lines of 1024 and beyond), at the shortest and longest lines, and
+4096-point columns; 1e-6 relative L2 against a 64-bit FFT: about 2^-24 per level of the transform."""
 import ctypes as C
 
 import pytest
